@@ -992,6 +992,59 @@ kf_status record_ms(cudaStream_t st, cudaEvent_t a, cudaEvent_t b, float* ms) {
     return KF_OK;
 }
 
+// Device scratch of one stage call, allocated and freed in the order of the call's stream, so
+// calls on several streams or threads never share it.  It comes from a memory pool of the
+// library's own, one per device (the device's default pool is the caller's), which keeps up to
+// kScratchKept bytes between calls -- a cudaMalloc and cudaFree per call cost tens of
+// microseconds and wait for the whole device -- and gives back what is above that at the next
+// synchronisation.
+constexpr int kScratchMaxDevices = 64;
+constexpr unsigned long long kScratchKept = 64ull << 20;
+std::mutex g_scratch_mu;
+cudaMemPool_t g_scratch_pool[kScratchMaxDevices] = {};
+
+cudaError_t scratch_pool(cudaMemPool_t* out) {
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= kScratchMaxDevices) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    if (!g_scratch_pool[dev]) {
+        cudaMemPoolProps props;
+        std::memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        e = cudaMemPoolCreate(&pool, &props);
+        if (e != cudaSuccess) return e;
+        unsigned long long keep = kScratchKept;
+        e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) { cudaMemPoolDestroy(pool); return e; }
+        g_scratch_pool[dev] = pool;
+    }
+    *out = g_scratch_pool[dev];
+    return cudaSuccess;
+}
+
+struct Scratch {
+    void* p = nullptr;
+    cudaStream_t st = nullptr;
+    cudaError_t take(size_t bytes, cudaStream_t s) {
+        cudaMemPool_t pool = nullptr;
+        cudaError_t e = scratch_pool(&pool);
+        if (e != cudaSuccess) return e;
+        st = s;
+        e = cudaMallocFromPoolAsync(&p, bytes, pool, s);
+        if (e != cudaSuccess) p = nullptr;
+        return e;
+    }
+    Scratch() = default;
+    ~Scratch() { if (p) cudaFreeAsync(p, st); }
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+};
+
 // event pair around a stage call when the caller asks for its time (the reference's
 // kernel:: wrappers all return elapsed milliseconds)
 struct StageTimer {
@@ -1715,19 +1768,12 @@ kf_status kf_fuse(const float* depth_m, int w, int h, const float cam_k[9], cons
     NvtxRange nvtx_("kf_fuse");
     if (!depth_m || !cam_k || !pose || w <= 0 || h <= 0) return KF_ERR_ARG;
     KF_TRY(check_volume(vol));
-    std::vector<float> xs(vol->n), zs(vol->n);
-    voxel_axes(vol->n, vol->width, xs.data(), zs.data());
-    float* d_ax = nullptr;
-    KF_CK(cudaMalloc(&d_ax, sizeof(float) * 2 * vol->n));
     cudaStream_t st = as_stream(stream);
-    cudaError_t e = cudaMemcpyAsync(d_ax, xs.data(), sizeof(float) * vol->n, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_ax + vol->n, zs.data(), sizeof(float) * vol->n, cudaMemcpyHostToDevice, st);
+    Scratch scratch;
+    KF_CK(scratch.take(stage_fuse_scratch(vol->n, w, h), st));
     StageTimer t(elapsed_ms, st);
-    if (e == cudaSuccess) e = stage_fuse(depth_m, w, h, cam_k, vol, pose, min_depth, max_depth, d_ax, d_ax + vol->n, st);
-    kf_status r = t.finish(e);
+    kf_status r = t.finish(stage_fuse(depth_m, w, h, cam_k, vol, pose, min_depth, max_depth, scratch.p, st));
     cudaStreamSynchronize(st);
-    cudaFree(d_ax);
     return r;
 }
 

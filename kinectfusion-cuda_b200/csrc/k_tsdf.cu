@@ -129,8 +129,9 @@ __device__ __forceinline__ bool block_culled(const FuseCtx& c, int x0, int j0, i
     float dm = 0.0f;
     for (int ty = ty0; ty <= ty1; ++ty)
         for (int tx = tx0; tx <= tx1; ++tx) dm = fmaxf(dm, __ldg(c.dmax + size_t(ty) * c.t16w + tx));
-    // every voxel meets either an invalid depth or d - z <= dm - zmin < -mu
-    return dm == 0.0f || zmin > dm + c.mu + 1e-4f;
+    // every voxel meets either an invalid depth or d - z <= dm - zmin < -mu (the margin also covers
+    // the sum's rounding where depths are in the thousands: a caller's maps in millimetres)
+    return dm == 0.0f || zmin > dm + c.mu + 1e-4f + 1e-6f * dm;
 }
 
 // block coordinates of fusion unit u of an n^3 volume (units: 32 x 8 x 8 blocks, x fastest)
@@ -545,38 +546,114 @@ cudaError_t launch_rebuild_bricks(const void* f, int fmt, int n, int* bmin, int*
 }
 
 // ---- stage fusion on a caller volume (kernel::fuse) ----
+//
+// The same cull, queue and fuse as a session's step, on scratch that the call brings.  The set-up
+// launch writes what a session keeps: the voxel axes and the depth map's 16 x 16 tile maxima.  Bound
+// by the queue's row updates, as a session's fusion.  One launch whose warps each tested and fused
+// 32 consecutive blocks, without the maxima, was bound by the few warps that held the frustum's
+// blocks: 808 us in the kernel at 640 x 480 into 512^3 f32, and up to 1 ms more per call in
+// cudaMalloc and cudaFree; the call now takes 83 us.
 
-__global__ void __launch_bounds__(256) fuse_stage_kernel(FuseCtx c) {
-    const int total = fuse_units(c.n);
+// the scratch of one call, carved from one allocation
+struct StageFuseScratch {
+    unsigned int* counters;   // [0] blocks queued, [1] items taken
+    float* xs;
+    float* zs;
+    float* dmax;
+    unsigned int* queue;
+};
+
+static size_t stage_fuse_layout(int n, int w, int h, char* base, StageFuseScratch* s) {
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~size_t(255); return base + o; };
+    StageFuseScratch r;
+    r.counters = reinterpret_cast<unsigned int*>(take(2 * sizeof(unsigned int)));
+    r.xs = reinterpret_cast<float*>(take(sizeof(float) * n));
+    r.zs = reinterpret_cast<float*>(take(sizeof(float) * n));
+    r.dmax = reinterpret_cast<float*>(take(sizeof(float) * size_t((w + 15) / 16) * ((h + 15) / 16)));
+    r.queue = reinterpret_cast<unsigned int*>(take(sizeof(unsigned int) * fuse_units(n)));
+    if (s) *s = r;
+    return at;
+}
+
+size_t stage_fuse_scratch(int n, int w, int h) { return stage_fuse_layout(n, w, h, nullptr, nullptr); }
+
+// Block 0: counters and voxel axes (voxel_axes on the host: every product and sum rounded on its
+// own, z accumulated step by step).  The other blocks: one warp per 16 x 16 tile of the depth map,
+// its largest valid depth.
+__global__ void __launch_bounds__(256) fuse_stage_setup_kernel(const float* depth, int w, int h, int n, float base,
+                                                               float res, StageFuseScratch s) {
+    const int tid = threadIdx.x;
+    if (blockIdx.x == 0) {
+        if (tid < 2) s.counters[tid] = 0u;
+        for (int i = tid; i < n; i += blockDim.x) s.xs[i] = __fadd_rn(base, __fmul_rn(float(i), res));
+        if (tid == 0) {
+            float z = __fsub_rn(base, res);
+            for (int k = 0; k < n; ++k) {
+                z = __fadd_rn(z, res);
+                s.zs[k] = z;
+            }
+        }
+        return;
+    }
+    const int lane = tid & 31, t16w = (w + 15) / 16, tiles = t16w * ((h + 15) / 16);
+    const int t = (blockIdx.x - 1) * 8 + (tid >> 5);
+    if (t >= tiles) return;
+    const int x = (t % t16w) * 16 + (lane & 15), y0 = (t / t16w) * 16 + (lane >> 4);
+    float m = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 16; k += 2) {
+        const float d = x < w && y0 + k < h ? __ldg(depth + size_t(y0 + k) * w + x) : 0.0f;
+        if (depth_valid(d)) m = fmaxf(m, d);
+    }
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    if (lane == 0) s.dmax[t] = m;
+}
+
+// one thread per block of the volume; survivors queued with one atomic per warp
+__global__ void __launch_bounds__(256) fuse_stage_cull_kernel(FuseCtx c, StageFuseScratch s) {
+    const int u = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    bool keep = false;
+    if (u < fuse_units(c.n)) {
+        int x0, j0, k0;
+        unit_origin(c.n, u, x0, j0, k0);
+        keep = !block_culled(c, x0, j0, k0);
+    }
+    const unsigned int m = __ballot_sync(0xffffffffu, keep);
+    if (m == 0) return;
+    unsigned int slot = 0;
+    if (lane == 0) slot = atomicAdd(s.counters, unsigned(__popc(m)));
+    slot = __shfl_sync(0xffffffffu, slot, 0);
+    if (keep) s.queue[slot + __popc(m & ((1u << lane) - 1u))] = unsigned(u);
+}
+
+__global__ void __launch_bounds__(256, 4) fuse_stage_kernel(FuseCtx c, StageFuseScratch s) {
     const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    // each warp tests 32 consecutive blocks (one per lane), then fuses the survivors together
-    for (int base = warp * 32; base < total; base += nwarps * 32) {
-        const int u = base + lane;
-        int x0 = 0, j0 = 0, k0 = 0;
-        bool keep = false;
-        if (u < total) {
-            unit_origin(c.n, u, x0, j0, k0);
-            keep = !block_culled(c, x0, j0, k0);
-        }
-        unsigned int m = __ballot_sync(0xffffffffu, keep);
-        while (m) {
-            const int q = __ffs(m) - 1;
-            m &= m - 1;
-            const int bx = __shfl_sync(0xffffffffu, x0, q), by = __shfl_sync(0xffffffffu, j0, q),
-                      bz = __shfl_sync(0xffffffffu, k0, q);
-            fuse_rows(c, bx, by, bz, 0, 64, lane);
-        }
+    const unsigned int blocks = __ldcg(s.counters);
+    const int split = fuse_split(blocks), rows = 64 / split;
+    const unsigned int items = blocks * unsigned(split);
+    while (true) {
+        unsigned int i = 0;
+        if (lane == 0) i = atomicAdd(s.counters + 1, 1u);
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i >= items) break;
+        const int part = int(i % unsigned(split));
+        int x0, j0, k0;
+        unit_origin(c.n, int(__ldcg(s.queue + i / unsigned(split))), x0, j0, k0);
+        fuse_rows(c, x0, j0, k0, part * rows, (part + 1) * rows, lane);
     }
 }
 
 cudaError_t stage_fuse(const float* depth, int w, int h, const float* k, const kf_volume* vol, const float* pose,
-                       float min_d, float max_d, const float* xs, const float* zs, cudaStream_t st) {
+                       float min_d, float max_d, void* scratch, cudaStream_t st) {
+    StageFuseScratch s;
+    stage_fuse_layout(vol->n, w, h, static_cast<char*>(scratch), &s);
     FuseCtx c;
     c.depth = depth;
-    c.dmax = nullptr;
-    c.t16w = c.t16h = 0;
+    c.dmax = s.dmax;
+    c.t16w = (w + 15) / 16;
+    c.t16h = (h + 15) / 16;
     c.w = w;
     c.h = h;
     c.fx = k[0]; c.fy = k[4]; c.cx = k[6]; c.cy = k[7];
@@ -586,15 +663,19 @@ cudaError_t stage_fuse(const float* depth, int w, int h, const float* k, const k
     c.fmt = vol->format;
     c.F = vol->f;
     c.W = vol->w;
-    c.xs = xs;
-    c.zs = zs;
+    c.xs = s.xs;
+    c.zs = s.zs;
     c.bmin = nullptr;
     // inverse of the rigid pose: R^T, -R^T t
     for (int col = 0; col < 3; ++col)
         for (int row = 0; row < 3; ++row) c.iR[col * 3 + row] = pose[row * 4 + col];
     for (int row = 0; row < 3; ++row)
         c.it[row] = -(c.iR[row] * pose[12] + c.iR[3 + row] * pose[13] + c.iR[6 + row] * pose[14]);
-    fuse_stage_kernel<<<148 * 8, 256, 0, st>>>(c);
+    const float res = vol->width / float(vol->n - 1), base = -vol->width * 0.5f;
+    const int tiles = c.t16w * c.t16h;
+    fuse_stage_setup_kernel<<<1 + (tiles + 7) / 8, 256, 0, st>>>(depth, w, h, vol->n, base, res, s);
+    fuse_stage_cull_kernel<<<(fuse_units(vol->n) + 255) / 256, 256, 0, st>>>(c, s);
+    fuse_stage_kernel<<<148 * 4, 256, 0, st>>>(c, s);
     return cudaGetLastError();
 }
 

@@ -115,8 +115,10 @@ struct DispMats {
 };
 cudaError_t stage_display(int mode, const void* src, int w, int h, const DispMats& m, float scale, unsigned int* out,
                           cudaStream_t st);
+// scratch: stage_fuse_scratch(n, w, h) bytes of device memory, used by this call's launches only
+size_t stage_fuse_scratch(int n, int w, int h);
 cudaError_t stage_fuse(const float* depth, int w, int h, const float* k, const kf_volume* vol, const float* pose,
-                       float min_d, float max_d, const float* xs, const float* zs, cudaStream_t st);
+                       float min_d, float max_d, void* scratch, cudaStream_t st);
 cudaError_t stage_icp_residuals(const float4* vmap, const float4* tv, const float4* tn, int w, int h,
                                 const float* Rp, const float* tp, const float* Rc, const float* tc, const float* k,
                                 float dist, float angle, float* A, float* b, cudaStream_t st);

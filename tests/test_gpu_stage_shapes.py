@@ -1,0 +1,62 @@
+"""Per-stage calls at the sizes where their work splits can go wrong -- the smallest and ragged
+volumes, frames that no tile divides, non-finite depths -- against the CPU oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def dev(torch, a):
+    a = np.ascontiguousarray(a)
+    return torch.from_numpy(a.view(np.int16) if a.dtype == np.uint16 else a).cuda()
+
+
+def depth_frames(kf, orc, w, h, unit):
+    """Two metre maps (times unit) of the synthetic loop with their poses, and K; the second map
+    holds zeros, a NaN and infinities too."""
+    from kfb200 import synth
+    cfg = kf.config_small(width=w, height=h, fx=262.5 * w / 320, fy=262.5 * w / 320, cx=w / 2 - 0.5, cy=h / 2 - 0.5)
+    imgs, poses = synth.sequence(cfg, 42, seed=9, kind=synth.LOOP)
+    maps, out = [], []
+    for i in (38, 41):
+        maps.append(orc.convert(imgs[i], 1e-3) * np.float32(unit))
+        p = poses[i].copy()
+        p[:3, 3] *= unit
+        out.append(p)
+    maps[1][h // 2, :3] = [np.nan, np.inf, -np.inf]
+    return cfg, maps, out, kf.level_intrinsics(cfg, 0)
+
+
+@pytest.mark.parametrize("n,w,h,fmt,unit", [(8, 33, 17, 0, 1.0), (40, 161, 119, 0, 1.0), (72, 160, 120, 1, 1.0),
+                                            (136, 321, 241, 0, 1.0), (136, 320, 240, 1, 1.0), (64, 320, 240, 0, 1000.0)])
+def test_fuse_shapes(kf, orc, cuda, n, w, h, fmt, unit):
+    """Two frames fused, at the oracle's state.  The second frame's values agree to 1e-3 of the
+    truncation distance (f16: plus the storage rounding 2^-10 of a value up to 1 and of the
+    weights' steps) except where a projection within float rounding of a pixel edge, the depth
+    range or the update limit picks otherwise: at most 0.5 % of the touched voxels, or three
+    voxels of the smallest volumes."""
+    _, maps, poses, k = depth_frames(kf, orc, w, h, unit)
+    width, mu = 2.0 * unit, max(0.03, 3.0 / n) * unit
+    f = np.full((n, n, n), 2.0, np.float32)
+    wt = np.zeros((n, n, n), np.float32)
+    rng = dict(min_d=0.4 * unit, max_d=6.0 * unit)
+    orc.fuse(maps[0], k, f, wt, width, mu, poses[0], prec=1, **rng)
+    if fmt:
+        f = f.astype(np.float16).astype(np.float32)
+        wq = np.minimum(np.rint(wt * kf.KF_WEIGHT_SCALE), 65535).astype(np.uint16)
+        wt = wq.astype(np.float32) / np.float32(kf.KF_WEIGHT_SCALE)
+        ft, wd = dev(cuda, f.astype(np.float16)), dev(cuda, wq)
+    else:
+        ft, wd = dev(cuda, f), dev(cuda, wt)
+    vol = kf.kernel.volume(ft, wd, width, mu, fmt=fmt)
+    kf.kernel.fuse(dev(cuda, maps[1]), vol, poses[1], k, min_depth=rng["min_d"], max_depth=rng["max_d"])
+    fo, wo = f.copy(), wt.copy()
+    orc.fuse(maps[1], k, fo, wo, width, mu, poses[1], prec=1, **rng)
+    gf = ft.cpu().numpy().astype(np.float32)
+    gw = wd.cpu().numpy()
+    gw = gw.view(np.uint16).astype(np.float32) / np.float32(kf.KF_WEIGHT_SCALE) if fmt else gw
+    touched = (wo != wt) | (gw != wt)
+    tol_f, tol_w = (2e-3, 0.5 / kf.KF_WEIGHT_SCALE + 1e-6) if fmt else (1e-3, 1e-5 * max(1.0, float(wo.max())))
+    bad = touched & ((np.abs(gf - fo) > tol_f) | (np.abs(gw - wo) > tol_w))
+    assert int(bad.sum()) <= max(3, 0.005 * int(touched.sum())), (int(bad.sum()), int(touched.sum()))
+    assert n == 8 or touched.sum() > 100
