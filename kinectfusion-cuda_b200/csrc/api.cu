@@ -1045,6 +1045,21 @@ struct Scratch {
     Scratch& operator=(const Scratch&) = delete;
 };
 
+int ray_queue_entries(int w, int h, bool bounds) {
+    const long long share = std::min(long_ray_entries((long long)w * h), (long long)(INT32_MAX / long_ray_bytes()));
+    return stage_raycast_queue(w, h, bounds, share);
+}
+
+// Scratch of a stage raycast.  A captured call takes none (its graph may be replayed while another
+// call runs, and an allocation inside it would restrict how the graph is used), nor does one that
+// finds no memory: stage_raycast then marches every ray in its own thread.
+void raycast_scratch(Scratch& scratch, int n, int longq_cap, cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone ||
+        scratch.take(stage_raycast_scratch(n, longq_cap), st) != cudaSuccess)
+        cudaGetLastError();
+}
+
 // event pair around a stage call when the caller asks for its time (the reference's
 // kernel:: wrappers all return elapsed milliseconds)
 struct StageTimer {
@@ -1659,8 +1674,11 @@ kf_status kf_render(kf_session* s, int mode, const float pose_in[16], uint8_t* r
     KF_CK(cudaStreamSynchronize(st));
     KF_CK(cudaMemsetAsync(sl.render_v, 0, size_t(w) * h * 16, st));
     KF_CK(cudaMemsetAsync(sl.render_n, 0, size_t(w) * h * 16, st));
+    const int cap = ray_queue_entries(w, h, true);
+    Scratch scratch;
+    raycast_scratch(scratch, 0, cap, st);
     KF_CK(stage_raycast(&vol, pose, ik, sl.render_v, sl.render_n, w, h, c.min_depth, c.max_depth, c.step_large,
-                        c.step_small, st, &bounds));
+                        c.step_small, scratch.p, cap, st, &bounds));
     DispMats m{};
     if (mode == KF_RENDER_NORMALS) {
         for (int cc = 0; cc < 3; ++cc)
@@ -1787,10 +1805,15 @@ kf_status kf_raycast(const kf_volume* vol, const float pose[16], const float inv
     if (!(step_large > step_small) || !(max_depth > min_depth) || !(max_depth < 1000.f) ||
         !(vol->mu * step_small > max_depth * 1e-6f))
         return KF_ERR_ARG;
-    StageTimer t(elapsed_ms, as_stream(stream));
+    cudaStream_t st = as_stream(stream);
+    const bool build = stage_raycast_builds_bounds(vol, w, h);
+    const int cap = ray_queue_entries(w, h, build);
+    Scratch scratch;
+    raycast_scratch(scratch, build ? vol->n : 0, cap, st);
+    StageTimer t(elapsed_ms, st);
     return t.finish(stage_raycast(vol, pose, inv_cam_k, reinterpret_cast<float4*>(vertex),
                                   reinterpret_cast<float4*>(normal), w, h, min_depth, max_depth, step_large,
-                                  step_small, as_stream(stream)));
+                                  step_small, scratch.p, cap, st));
 }
 
 kf_status kf_construct_icp_residuals(const float* vertex, const float* target_vertex, const float* target_normal, int w,

@@ -28,6 +28,9 @@
 //   - Long rays: a second kernel marches each queued ray with a whole warp, 32 consecutive
 //     samples per round (64 after a round in which nothing changed), taking the first sample
 //     (in order) that changes the state.
+#include <algorithm>
+#include <cmath>
+
 #include "kf_host.h"
 
 namespace kf {
@@ -585,8 +588,15 @@ __device__ __forceinline__ void write_miss(const SessionDev* S, int level, int i
     S->pn[level][size_t(j) * w + i] = make_float4(0.f, 0.f, 0.f, kInvalid);
 }
 
+// where lanes hand over the rays they do not finish
+struct RayQueue {
+    LongRay* rays;
+    unsigned int* count;
+    int cap;
+};
+
 template <class TF, class Cnt, bool kEager>
-__device__ void serial_ray(const EngineView& v, const SessionDev* S, int s, const float* m, F3 o, int level, int i,
+__device__ void serial_ray(const RayQueue& rq, const SessionDev* S, int s, const float* m, F3 o, int level, int i,
                            int j, int budget, Cnt& cnt) {
     const TF* f = static_cast<const TF*>(S->tf);
     RayGeo g;
@@ -599,9 +609,9 @@ __device__ void serial_ray(const EngineView& v, const SessionDev* S, int s, cons
     cnt.add(kCntRays, 1u);
     float precise = 0.0f;
     if (!march_serial<TF, Cnt, kEager>(S, g, f, st, budget, precise, cnt)) {
-        const unsigned int slot = atomicAdd(&v.counters[6], 1u);
-        if (slot < unsigned(v.longq_cap)) {
-            v.longq[slot] = LongRay{s, level, i, j, st, g};
+        const unsigned int slot = atomicAdd(rq.count, 1u);
+        if (slot < unsigned(rq.cap)) {
+            rq.rays[slot] = LongRay{s, level, i, j, st, g};
             cnt.add(kCntQueued, 1u);
             return;
         }
@@ -621,6 +631,7 @@ __global__ void __launch_bounds__(256, kBlocksPerSm) raycast_kernel(EngineView v
     const int budget = v.tb->ray_budget;
     const int tw = v.tb->ray_tw;
     const int lx = lane % tw, ly = lane / tw;
+    const RayQueue rq{v.longq, v.counters + 6, v.longq_cap};
     while (true) {
         int t = 0;
         if (lane == 0) t = int(atomicAdd(&v.counters[0], 1u));
@@ -637,9 +648,9 @@ __global__ void __launch_bounds__(256, kBlocksPerSm) raycast_kernel(EngineView v
         F3 o;
         ray_matrix(S, Lv, m, o);
         if (S->fmt == KF_TSDF_F16U16)
-            serial_ray<__half, MarchCount<kCount>, kBlocksPerSm == 3>(v, S, T.s, m, o, T.level, i, j, budget, cnt);
+            serial_ray<__half, MarchCount<kCount>, kBlocksPerSm == 3>(rq, S, T.s, m, o, T.level, i, j, budget, cnt);
         else
-            serial_ray<float, MarchCount<kCount>, kBlocksPerSm == 3>(v, S, T.s, m, o, T.level, i, j, budget, cnt);
+            serial_ray<float, MarchCount<kCount>, kBlocksPerSm == 3>(rq, S, T.s, m, o, T.level, i, j, budget, cnt);
     }
     cnt.flush(v.ray_counts);
 }
@@ -695,13 +706,157 @@ cudaError_t launch_raycast(const EngineView& v, int grid, cudaStream_t st, bool 
 
 int ray_count_slots() { return kRayCounts; }
 
-// ---- stage kernel: kernel::raycast on a caller volume ----
+// ---- stage: kernel::raycast on a caller volume, and kf_render on a session's ----
+//
+// A caller's volume has no brick bounds, so the call makes them: one read of the distances of
+// every block that the rays can reach, then the session's march -- 8 x 4-ray tiles, a lane budget,
+// long rays by whole warps.  Bound by that read (HBM) and then by the march's instructions.  One
+// thread per ray without skipping, as the reference marches, was bound by its longest rays (about
+// 2,800 samples one after another): 640 x 480 rays in 512^3 f32 took 732 us in the kernel, now
+// 180; kf_render's on a session's bounds 427 us, now about 200.
 
 struct RayStage {
-    float m[9];
+    float m[9];      // R K^-1 (column-major)
     float o[3];
+    float inv[9];    // its inverse: (p - o) to (pixel * t, t); valid when has_inv
+    int has_inv;
 };
 
+// the scratch of one call, carved from one allocation
+struct StageRayScratch {
+    unsigned int* counters;   // [0] ray tiles, [1] long rays queued, [2] long rays taken
+    int* bmin;
+    int* bdil;
+    int* sdil;
+    LongRay* longq;
+    int longq_cap;
+};
+
+static size_t stage_ray_layout(int n, int longq_cap, char* base, StageRayScratch* s) {
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~size_t(255); return base + o; };
+    const size_t nb = size_t(n / 8), ns = (nb + 3) / 4;   // n = 0: no bounds
+    StageRayScratch r;
+    r.counters = reinterpret_cast<unsigned int*>(take(4 * sizeof(unsigned int)));
+    r.bmin = reinterpret_cast<int*>(take(sizeof(int) * nb * nb * nb));
+    r.bdil = reinterpret_cast<int*>(take(sizeof(int) * nb * nb * nb));
+    r.sdil = reinterpret_cast<int*>(take(sizeof(int) * ns * ns * ns));
+    r.longq = reinterpret_cast<LongRay*>(take(sizeof(LongRay) * size_t(longq_cap)));
+    r.longq_cap = longq_cap;
+    if (s) *s = r;
+    return at;
+}
+
+size_t stage_raycast_scratch(int n, int longq_cap) { return stage_ray_layout(n, longq_cap, nullptr, nullptr); }
+
+__device__ __forceinline__ float min4(float4 v) { return fminf(fminf(v.x, v.y), fminf(v.z, v.w)); }
+__device__ __forceinline__ float min_half2(unsigned int bits) {
+    const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&bits));
+    return fminf(v.x, v.y);
+}
+__device__ __forceinline__ int order_key(float x) {   // order-preserving int of a float of either sign
+    const int i = __float_as_int(x);
+    return i >= 0 ? i : (i ^ 0x7fffffff);
+}
+
+// bmin of every 8^3 brick, one warp per 32 x 8 x 8 block.  A block that no ray of the image can
+// sample -- its box, widened by the voxel that a sample's taps reach, lies outside one of the six
+// planes of the rays' frustum -- is not read; its bound says 2, which no sample sees.  Else the
+// warp reads 128-byte (f32) or 64-byte (f16) rows with all its 16-byte loads in flight.
+template <class TF>
+__global__ void __launch_bounds__(256) stage_bounds_kernel(const TF* f, int n, float vol_w, RayStage rs, int w, int h,
+                                                           float min_d, float max_d, StageRayScratch s) {
+    if (blockIdx.x == 0 && threadIdx.x < 4) s.counters[threadIdx.x] = 0u;
+    const int lane = threadIdx.x & 31, u = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int ux = (n + 31) >> 5, uy = n >> 3, nb = n >> 3;
+    if (u >= ux * uy * uy) return;
+    const int x0 = (u % ux) * 32, y0 = ((u / ux) % uy) * 8, z0 = (u / (ux * uy)) * 8;
+    int* out = s.bmin + (size_t(z0 >> 3) * nb + (y0 >> 3)) * nb + (x0 >> 3);
+    const int bricks = min(4, nb - (x0 >> 3));
+    if (rs.has_inv) {
+        // lanes 0-7 (and their copies) hold the widened box's corners
+        const float to_m = vol_w / float(n), mid = 0.5f * float(n) - 0.5f;
+        const float px = ((lane & 1 ? float(min(x0 + 32, n)) + 0.05f : float(x0) - 1.05f) - mid) * to_m - rs.o[0];
+        const float py = ((lane & 2 ? float(y0 + 8) + 0.05f : float(y0) - 1.05f) - mid) * to_m - rs.o[1];
+        const float pz = ((lane & 4 ? float(z0 + 8) + 0.05f : float(z0) - 1.05f) - mid) * to_m - rs.o[2];
+        const F3 q = mv3(rs.inv, F3{px, py, pz});   // (i t, j t, t); samples have i in [.5, w - .5]
+        const unsigned int all = 0xffffffffu;
+        if (__all_sync(all, q.x < 0.f) || __all_sync(all, q.x > float(w) * q.z) || __all_sync(all, q.y < 0.f) ||
+            __all_sync(all, q.y > float(h) * q.z) || __all_sync(all, q.z < 0.999f * min_d) ||
+            __all_sync(all, q.z > 1.001f * max_d)) {
+            if (lane < bricks) out[lane] = 0x40000000;   // key of 2.0f
+            return;
+        }
+    }
+    float m = 3.0e38f;
+    if constexpr (sizeof(TF) == 4) {
+        const int x = x0 + 4 * (lane & 7);
+        if (x < n) {
+            const float4* p = reinterpret_cast<const float4*>(f + (size_t(z0) * n + y0 + (lane >> 3)) * n + x);
+            const size_t row = size_t(n) / 4, slice = size_t(n) * row;   // n % 8 == 0
+            float4 v[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] = __ldg(p + (k >> 1) * slice + (k & 1) * 4 * row);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) m = fminf(m, min4(v[k]));
+        }
+        m = fminf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+        m = fminf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+        m = fminf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+        if ((lane & 0x19) == 0 && x < n) out[lane >> 1] = order_key(m);
+    } else {
+        const int x = x0 + 8 * (lane & 3);
+        if (x < n) {
+            const uint4* p = reinterpret_cast<const uint4*>(f + (size_t(z0) * n + y0 + (lane >> 2)) * n + x);
+            const size_t slice = size_t(n) * n / 8;
+            uint4 v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = __ldg(p + k * slice);
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                m = fminf(m, fminf(fminf(min_half2(v[k].x), min_half2(v[k].y)), fminf(min_half2(v[k].z), min_half2(v[k].w))));
+        }
+        m = fminf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+        m = fminf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+        m = fminf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+        if (lane < 4 && x < n) out[lane] = order_key(m);
+    }
+}
+
+// each warp pulls 8 x 4-ray tiles, as in a session's raycast
+template <class TF>
+__global__ void __launch_bounds__(256, 3) raycast_tiles_stage_kernel(const __grid_constant__ SessionDev S,
+                                                                     const __grid_constant__ RayStage rs, int w, int h,
+                                                                     int budget, StageRayScratch sc) {
+    MarchCount<false> cnt;
+    const int lane = threadIdx.x & 31, tx = (w + 7) / 8, ntiles = tx * ((h + 3) / 4);
+    const RayQueue rq{sc.longq, sc.counters + 1, sc.longq_cap};
+    while (true) {
+        int t = 0;
+        if (lane == 0) t = int(atomicAdd(sc.counters, 1u));
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t >= ntiles) break;
+        const int i = (t % tx) * 8 + (lane & 7), j = (t / tx) * 4 + (lane >> 3);
+        if (i >= w || j >= h) continue;
+        serial_ray<TF, MarchCount<false>, true>(rq, &S, 0, rs.m, F3{rs.o[0], rs.o[1], rs.o[2]}, 0, i, j, budget, cnt);
+    }
+}
+
+template <class TF>
+__global__ void __launch_bounds__(256) raycast_long_stage_kernel(const __grid_constant__ SessionDev S, StageRayScratch sc) {
+    MarchCount<false> cnt;
+    const int lane = threadIdx.x & 31;
+    const int count = min(int(sc.counters[1]), sc.longq_cap);
+    while (true) {
+        int idx = 0;
+        if (lane == 0) idx = int(atomicAdd(sc.counters + 2, 1u));
+        idx = __shfl_sync(0xffffffffu, idx, 0);
+        if (idx >= count) break;
+        coop_ray<TF>(&S, sc.longq[idx], lane, cnt);
+    }
+}
+
+// one thread per ray, no scratch: for a call under stream capture, or one that finds no memory
 template <class TF>
 __global__ void raycast_stage_kernel(SessionDev S, RayStage rs, int w, int h) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -720,9 +875,61 @@ __global__ void raycast_stage_kernel(SessionDev S, RayStage rs, int w, int h) {
     finish_ray(&S, g, f, 0, i, j, precise, st, cnt);
 }
 
+// Bounds cost a read of the visible volume whatever the image, and the march without them costs in
+// proportion to the rays, in volumes of every size (a finer volume has more samples per ray).  Both
+// ways measured, us, image x volume, without / with bounds: 320x240 in 128^3 f32 45 / 58, in 256^3
+// 69 / 79, in 512^3 138 / 166; 640x480 in 128^3 73 / 75, in 256^3 111 / 102, in 512^3 210 / 179
+// (f16 202 / 148).  The line lies between the two images.
+constexpr long long kBoundsRays = 160000;
+
+bool stage_raycast_builds_bounds(const kf_volume* vol, int w, int h) {
+    return (long long)w * h >= kBoundsRays && reinterpret_cast<uintptr_t>(vol->f) % 16 == 0;   // vector reads
+}
+
+// Without bounds a lane's budget is short for small images, whose few warps leave the GPU idle
+// while a lane marches (80x60 in 512^3 f32: 53 us at 24, 63 at 64), and long enough to reach most
+// surfaces for larger ones (320x240 in 512^3 f32: 203 us at 24, 138 at 64).
+static int budget_without_bounds(int w, int h) { return (long long)w * h <= 24000 ? 24 : 64; }
+
+// Every ray of a march without bounds may outlast its budget, and a ray that finds the queue full
+// marches on alone, several times slower; with bounds few do (long_ray_entries).
+int stage_raycast_queue(int w, int h, bool bounds, long long share) {
+    const long long rays = (long long)w * h;
+    return int(bounds ? share : std::max(share, std::min(rays, 1LL << 18)));
+}
+
+template <class TF>
+static cudaError_t launch_stage(SessionDev& S, const RayStage& rs, int w, int h, bool build, void* scratch,
+                                int longq_cap, cudaStream_t st) {
+    if (!scratch) {
+        const dim3 blk(8, 8), grd((w + 7) / 8, (h + 7) / 8);
+        raycast_stage_kernel<TF><<<grd, blk, 0, st>>>(S, rs, w, h);
+        return cudaGetLastError();
+    }
+    StageRayScratch sc;
+    stage_ray_layout(build ? S.n : 0, longq_cap, static_cast<char*>(scratch), &sc);
+    if (build) {
+        S.nb = S.n / 8;
+        S.ns = (S.nb + 3) / 4;
+        S.bdil = sc.bdil;
+        S.sdil = sc.sdil;
+        stage_bounds_kernel<TF><<<(fuse_units(S.n) + 7) / 8, 256, 0, st>>>(static_cast<const TF*>(S.tf), S.n, S.vol_w, rs,
+                                                                           w, h, S.min_d, S.max_d, sc);
+        cudaError_t e = launch_widen_bricks(sc.bmin, sc.bdil, sc.sdil, S.n, st);
+        if (e != cudaSuccess) return e;
+    } else {
+        cudaError_t e = cudaMemsetAsync(sc.counters, 0, 4 * sizeof(unsigned int), st);
+        if (e != cudaSuccess) return e;
+    }
+    const int tiles = ((w + 7) / 8) * ((h + 3) / 4), grid = std::min(148 * 6, (tiles + 7) / 8);
+    raycast_tiles_stage_kernel<TF><<<grid, 256, 0, st>>>(S, rs, w, h, S.bdil ? kSerialBudgetSingle : budget_without_bounds(w, h), sc);
+    raycast_long_stage_kernel<TF><<<148 * 4, 256, 0, st>>>(S, sc);
+    return cudaGetLastError();
+}
+
 cudaError_t stage_raycast(const kf_volume* vol, const float* pose, const float* ik, float4* vtx, float4* nrm, int w,
-                          int h, float min_d, float max_d, float step_l, float step_s, cudaStream_t st,
-                          const SessionDev* bounds) {
+                          int h, float min_d, float max_d, float step_l, float step_s, void* scratch, int longq_cap,
+                          cudaStream_t st, const SessionDev* bounds) {
     SessionDev S{};
     if (bounds) {   // a session's brick bounds: the same samples, skipping exactly as the pipeline
         S.bdil = bounds->bdil;
@@ -759,12 +966,22 @@ cudaError_t stage_raycast(const kf_volume* vol, const float* pose, const float* 
     rs.o[0] = pose[12];
     rs.o[1] = pose[13];
     rs.o[2] = pose[14];
-    dim3 blk(8, 8), grd((w + 7) / 8, (h + 7) / 8);
-    if (vol->format == KF_TSDF_F16U16)
-        raycast_stage_kernel<__half><<<grd, blk, 0, st>>>(S, rs, w, h);
-    else
-        raycast_stage_kernel<float><<<grd, blk, 0, st>>>(S, rs, w, h);
-    return cudaGetLastError();
+    // the inverse (adjugate over determinant), only to place the frustum's planes
+    {
+        const float* m = rs.m;
+        const double a = m[0], b = m[3], c = m[6], d = m[1], e = m[4], f = m[7], g = m[2], hh = m[5], i = m[8];
+        const double det = a * (e * i - f * hh) - b * (d * i - f * g) + c * (d * hh - e * g);
+        const double adj[9] = {e * i - f * hh, f * g - d * i, d * hh - e * g, c * hh - b * i, a * i - c * g,
+                               b * g - a * hh, b * f - c * e, c * d - a * f, a * e - b * d};
+        rs.has_inv = 1;
+        for (int q = 0; q < 9; ++q) {
+            rs.inv[q] = float(adj[q] / det);
+            if (!std::isfinite(rs.inv[q])) rs.has_inv = 0;
+        }
+    }
+    const bool build = !bounds && stage_raycast_builds_bounds(vol, w, h);
+    if (vol->format == KF_TSDF_F16U16) return launch_stage<__half>(S, rs, w, h, build, scratch, longq_cap, st);
+    return launch_stage<float>(S, rs, w, h, build, scratch, longq_cap, st);
 }
 
 }  // namespace kf

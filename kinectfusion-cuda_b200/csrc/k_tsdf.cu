@@ -517,22 +517,27 @@ __global__ void rebuild_bricks_kernel(const TF* f, int n, int* bmin) {
     }
 }
 
-__global__ void dilate_one_kernel(const int* bmin, int* bdil, int nb) {
-    const long long total = (long long)nb * nb * nb;
-    for (long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x; b < total; b += (long long)gridDim.x * blockDim.x)
-        dilate_brick(bmin, bdil, nb, int(b));
-}
-
-__global__ void superbrick_one_kernel(const int* bmin, int* sdil, int nb) {
-    const int ns = (nb + 3) / 4;
-    const long long total = (long long)ns * ns * ns;
-    const int lane = threadIdx.x & 31;
-    const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long b = warp; b < total; b += nwarps) {
-        const int k = superbrick_bound(bmin, nb, int(b % ns), int((b / ns) % ns), int(b / ((long long)ns * ns)), lane);
+// bdil by the first blocks (one thread per brick), sdil by the rest (one warp per super-brick)
+__global__ void __launch_bounds__(256) widen_kernel(const int* bmin, int* bdil, int* sdil, int nb, int dilate_blocks) {
+    const int total = nb * nb * nb;
+    if (int(blockIdx.x) < dilate_blocks) {
+        for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < total; b += dilate_blocks * blockDim.x)
+            dilate_brick(bmin, bdil, nb, b);
+        return;
+    }
+    const int ns = (nb + 3) / 4, lane = threadIdx.x & 31;
+    const int warp = ((blockIdx.x - dilate_blocks) * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = ((gridDim.x - dilate_blocks) * blockDim.x) >> 5;
+    for (int b = warp; b < ns * ns * ns; b += nwarps) {
+        const int k = superbrick_bound(bmin, nb, b % ns, (b / ns) % ns, b / (ns * ns), lane);
         if (lane == 0) sdil[b] = k;
     }
+}
+
+cudaError_t launch_widen_bricks(const int* bmin, int* bdil, int* sdil, int n, cudaStream_t st) {
+    const int nb = n / 8;
+    widen_kernel<<<148 * 8, 256, 0, st>>>(bmin, bdil, sdil, nb, 148 * 4);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_rebuild_bricks(const void* f, int fmt, int n, int* bmin, int* bdil, int* sdil, cudaStream_t st) {
@@ -540,9 +545,7 @@ cudaError_t launch_rebuild_bricks(const void* f, int fmt, int n, int* bmin, int*
         rebuild_bricks_kernel<<<148 * 8, 256, 0, st>>>(static_cast<const __half*>(f), n, bmin);
     else
         rebuild_bricks_kernel<<<148 * 8, 256, 0, st>>>(static_cast<const float*>(f), n, bmin);
-    dilate_one_kernel<<<148 * 4, 256, 0, st>>>(bmin, bdil, n / 8);
-    superbrick_one_kernel<<<148 * 4, 256, 0, st>>>(bmin, sdil, n / 8);
-    return cudaGetLastError();
+    return launch_widen_bricks(bmin, bdil, sdil, n, st);
 }
 
 // ---- stage fusion on a caller volume (kernel::fuse) ----

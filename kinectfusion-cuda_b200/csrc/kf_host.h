@@ -86,6 +86,7 @@ cudaError_t launch_fuse(const EngineView& v, int grid, cudaStream_t st);
 cudaError_t launch_fuse_vis(const EngineView& v, int grid, cudaStream_t st);
 // bounds = key(2), the initial distance; rebuild recomputes them exactly from a loaded volume
 cudaError_t launch_init_bricks(int* bmin, int* bdil, int* sdil, int n, cudaStream_t st);
+cudaError_t launch_widen_bricks(const int* bmin, int* bdil, int* sdil, int n, cudaStream_t st);
 cudaError_t launch_rebuild_bricks(const void* f, int fmt, int n, int* bmin, int* bdil, int* sdil, cudaStream_t st);
 int icp_max_grid(int num_sms);
 int long_ray_bytes();
@@ -103,10 +104,15 @@ cudaError_t stage_bilateral(const float* in, float* out, int w, int h, float ss,
 cudaError_t stage_down_sample(const float* in, float* out, int wo, int ho, float sr, cudaStream_t st);
 cudaError_t stage_vertex(const float* d, float4* v, int w, int h, const float* ik, cudaStream_t st);
 cudaError_t stage_normal(const float4* v, float4* n, int w, int h, cudaStream_t st);
-// bounds (optional): a session whose brick bounds the march may use to skip
+// bounds (optional): a session whose brick bounds the march may use to skip.  scratch:
+// stage_raycast_scratch bytes of device memory with room for longq_cap long rays (n: the volume's
+// size when the call builds bounds, else 0), or null to march every ray in its own thread.
+bool stage_raycast_builds_bounds(const kf_volume* vol, int w, int h);
+int stage_raycast_queue(int w, int h, bool bounds, long long share);   // share: a session's entries
+size_t stage_raycast_scratch(int n, int longq_cap);
 cudaError_t stage_raycast(const kf_volume* vol, const float* pose, const float* ik, float4* vtx, float4* nrm, int w,
-                          int h, float min_d, float max_d, float step_l, float step_s, cudaStream_t st,
-                          const SessionDev* bounds = nullptr);
+                          int h, float min_d, float max_d, float step_l, float step_s, void* scratch, int longq_cap,
+                          cudaStream_t st, const SessionDev* bounds = nullptr);
 // headless display (project/src/display.cu): RGBA8 images
 constexpr int kDisplayNormals = 0, kDisplayShading = 1, kDisplayFloat = 2;
 struct DispMats {

@@ -60,3 +60,64 @@ def test_fuse_shapes(kf, orc, cuda, n, w, h, fmt, unit):
     bad = touched & ((np.abs(gf - fo) > tol_f) | (np.abs(gw - wo) > tol_w))
     assert int(bad.sum()) <= max(3, 0.005 * int(touched.sum())), (int(bad.sum()), int(touched.sum()))
     assert n == 8 or touched.sum() > 100
+
+
+def plain_raycast(kf, cuda, vol, pose, ik, v, n, step, depths):
+    """kf_raycast under stream capture, replayed once: a captured call marches every ray in its own
+    thread, without bounds, scratch or queue."""
+    import ctypes
+    h, w = v.shape[:2]
+    s = cuda.cuda.Stream()
+    cuda.cuda.synchronize()
+    g = cuda.cuda.CUDAGraph()
+    with cuda.cuda.graph(g, stream=s):
+        st = kf.lib.kf_raycast(ctypes.byref(vol), kf.to_colmajor(pose), kf.to_colmajor(ik),
+                               ctypes.c_void_p(v.data_ptr()), w, h, ctypes.c_void_p(n.data_ptr()), w, h, depths[0],
+                               depths[1], step[0], step[1], ctypes.c_void_p(s.cuda_stream), None)
+        assert st == kf.KF_OK
+    g.replay()
+    cuda.cuda.synchronize()
+
+
+VIEWS = {"loop": None, "inside": (0.1, 0.1, 0.35), "away": (3.0, 0.0, 4.0), "mirrored": None}
+
+
+@pytest.mark.parametrize("n,w,h,fmt,view", [(8, 33, 17, 0, "loop"), (40, 161, 119, 1, "loop"), (72, 401, 401, 0, "loop"),
+                                            (136, 500, 330, 1, "loop"), (136, 500, 330, 0, "inside"),
+                                            (136, 500, 330, 0, "away"), (136, 500, 330, 0, "mirrored"),
+                                            (136, 500, 331, 0, "unaligned"), (512, 640, 480, 0, "loop"),
+                                            (256, 160, 120, 1, "inside")])
+def test_raycast_paths_agree(kf, orc, cuda, n, w, h, fmt, view):
+    """A call with scratch (bounds from one read of the visible volume, or none; ray tiles; long
+    rays by warps) gives the maps of the call without any, bit for bit: skipping and queueing
+    change which samples are evaluated where, not a sample's value or its test."""
+    _, maps, poses, k = depth_frames(kf, orc, w, h, 1.0)
+    width, mu = 2.0, max(0.01, 3.0 / n)
+    f = cuda.full((n, n, n), 2.0, device="cuda")
+    wt = cuda.zeros((n, n, n), device="cuda")
+    vol = kf.kernel.volume(f, wt, width, mu)
+    for m, p in zip(maps, poses):
+        kf.kernel.fuse(dev(cuda, m), vol, p, k)
+    if fmt:
+        f, wt = f.half(), wt.short()
+        vol = kf.kernel.volume(f, wt, width, mu, fmt=fmt)
+    if view == "unaligned":
+        room = cuda.zeros(n ** 3 + 1, device="cuda")
+        room[1:] = f.reshape(-1)
+        vol.f = room.data_ptr() + 4
+    pose, depths = poses[1].copy(), (0.4, 6.0)
+    if view == "inside":
+        pose[:3, 3] = VIEWS[view]
+        depths = (0.0, 6.0)
+    elif view == "away":
+        pose[:3, 3] = VIEWS[view]
+    ik = np.linalg.inv(k.astype(np.float64)).astype(np.float32)
+    if view == "mirrored":
+        ik = ik @ np.array([[-1, 0, w], [0, 1, 0], [0, 0, 1]], np.float32)
+    out = [[cuda.full((h, w, 4), 7.0, device="cuda") for _ in range(2)] for _ in range(2)]
+    kf.kernel.raycast(vol, pose, ik, *out[0], min_depth=depths[0], max_depth=depths[1])
+    plain_raycast(kf, cuda, vol, pose, ik, *out[1], (1.99, 0.1), depths)
+    for a, b in zip(*out):
+        assert cuda.equal(a.view(cuda.int32), b.view(cuda.int32))
+    hits = float((out[0][0][..., 3] == -1).float().mean())
+    assert hits > 0.05 or n == 8 or view in ("away", "inside"), hits
