@@ -98,6 +98,7 @@ size_t footprint(const kf_config& c) {
     const size_t nb = size_t(c.volume_n / 8), ns = (nb + 3) / 4;
     b += nb * nb * nb * 2 * sizeof(int) + ns * ns * ns * sizeof(int);
     b += sizeof(float) * size_t((c.width + 15) / 16) * ((c.height + 15) / 16);
+    b += sizeof(unsigned int) * range_words(c.width, c.height);   // the raycast's depth ranges
     if (c.vis_volume_n) {   // the visualization volume: grid, axes, brick and super-brick bounds
         const size_t vn = size_t(c.vis_volume_n), vnb = vn / 8, vns = (vnb + 3) / 4;
         b += vn * vn * vn * (c.tsdf_format == KF_TSDF_F16U16 ? 4 : 8) + sizeof(float) * 2 * vn;
@@ -347,6 +348,10 @@ kf_status slot_create(Slot& s, const kf_config& c, cudaStream_t st = nullptr) {
     KF_ALLOC(d.bmin, int*, sizeof(int) * size_t(nbricks));
     KF_ALLOC(d.bdil, int*, sizeof(int) * size_t(nbricks));
     KF_ALLOC(d.sdil, int*, sizeof(int) * size_t(nsuper));
+    if (c.volume_n >= kRangeMinN)
+        KF_ALLOC(d.range, unsigned int*, sizeof(unsigned int) * range_words(c.width, c.height));
+    d.rgw = (c.width + kRangeTile - 1) / kRangeTile;
+    d.rgh = (c.height + kRangeTile - 1) / kRangeTile;
     std::vector<float> vhx, vhz;   // alive until the stream sync below
     if (c.vis_volume_n) {
         VisDev& V = d.vis;
@@ -507,11 +512,10 @@ struct Engine {
     float* d_partials = nullptr;
     int4* d_icp_sched = nullptr;
     float* d_icp_mats = nullptr;
-    // one block [OutDev x cap | GridSync | counters]: a step clears the wait record and the
-    // counters with one memset, and a caller that reads the results copies them with one copy
+    // one block [OutDev x cap | GridSync | counters]: the start of a step clears the wait record and
+    // the counters at once, and a caller that reads the results copies them with one copy
     GridSync* d_sync = nullptr;
     unsigned int* d_ctr = nullptr;
-    static constexpr int kCounters = 12;
     size_t out_bytes() const { return sizeof(OutDev) * cap + sizeof(GridSync); }
     int cap_pre = 0, cap_ray = 0, cap_it = 0, cap_part = 0;
     // long-ray queue of the raycaster (bytes; entries = bytes / long_ray_bytes())
@@ -523,6 +527,7 @@ struct Engine {
     unsigned int* d_vfuseq = nullptr;
     int cap_vfuseq = 0;
     bool has_vis = false;      // some slot has a visualization volume: the step fuses it too
+    bool has_range = false;    // some slot's raycast takes depth ranges: the step makes them
     unsigned long long* d_ray_counts = nullptr;   // debug mode KF_DEBUG_COUNTERS: raycast work counts
     bool count_rays = false;
     // work-list entries reserved ahead for sessions not open yet (reserve_work)
@@ -751,6 +756,7 @@ struct Engine {
         std::vector<long long> fprefix(cap + 1, 0), vfprefix(cap + 1, 0);
         std::vector<SessionDev> sess(cap);
         int max_levels = 1;
+        bool range = false;
         for (int s = 0; s < cap; ++s) {
             const Slot& sl = slots[s];
             fprefix[s + 1] = fprefix[s];
@@ -759,6 +765,7 @@ struct Engine {
             sess[s] = sl.d;
             const kf_config& c = sl.cfg;
             max_levels = std::max(max_levels, c.levels);
+            range |= sl.d.range != nullptr;
             if (!sl.external) {
                 for (int y = 0; y < c.height; y += kPreTileSize)
                     for (int x = 0; x < c.width; x += kPreTileSize) pre.push_back(PreTile{s, x, y});
@@ -812,6 +819,8 @@ struct Engine {
         const bool vis = vfprefix[cap] > 0;
         if (vis != has_vis) graph_dirty = true;   // the step launches the visualization fusion or not
         has_vis = vis;
+        if (range != has_range) graph_dirty = true;   // the step makes depth ranges or not
+        has_range = range;
         KF_TRY(grow(d_pre, cap_pre, std::max<int>(1, int(pre.size()))));
         KF_TRY(grow(d_ray, cap_ray, std::max<int>(1, int(ray.size()))));
         KF_TRY(grow(d_itiles, cap_it, std::max<int>(1, int(all.size()))));
@@ -852,7 +861,6 @@ struct Engine {
     // the per-step sequence
     kf_status record(cudaStream_t st) {
         const EngineView v = view();
-        KF_CK(cudaMemsetAsync(d_sync, 0, sizeof(GridSync) + sizeof(unsigned int) * kCounters, st));
         if (count_rays) KF_CK(cudaMemsetAsync(d_ray_counts, 0, sizeof(unsigned long long) * ray_count_slots(), st));
         if (profile) KF_CK(cudaEventRecordWithFlags(ev[0], st, cudaEventRecordExternal));
         const bool fork = stages[0] && stages[1];
@@ -870,6 +878,13 @@ struct Engine {
             NvtxRange r("kf.preprocess");
             if (stages[0]) KF_CK(launch_preprocess(v, shape.grid_pre, st));
             if (profile) KF_CK(cudaEventRecordWithFlags(ev[1], st, cudaEventRecordExternal));
+        }
+        // clear the wait record and the counters; the depth-range launch does it on the way
+        if (has_range) {
+            const int units_grid = int(std::min<long long>((tb.fuse_total + 255) / 256, sms * 4));
+            KF_CK(launch_ray_range(v, cap == 1 ? units_grid : sms * 4, st));
+        } else {
+            KF_CK(cudaMemsetAsync(d_sync, 0, sizeof(GridSync) + sizeof(unsigned int) * kCounters, st));
         }
         {
             NvtxRange r("kf.raycast");
@@ -1053,10 +1068,10 @@ int ray_queue_entries(int w, int h, bool bounds) {
 // Scratch of a stage raycast.  A captured call takes none (its graph may be replayed while another
 // call runs, and an allocation inside it would restrict how the graph is used), nor does one that
 // finds no memory: stage_raycast then marches every ray in its own thread.
-void raycast_scratch(Scratch& scratch, int n, int longq_cap, cudaStream_t st) {
+void raycast_scratch(Scratch& scratch, int n, int w, int h, int longq_cap, cudaStream_t st) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone ||
-        scratch.take(stage_raycast_scratch(n, longq_cap), st) != cudaSuccess)
+        scratch.take(stage_raycast_scratch(n, w, h, longq_cap), st) != cudaSuccess)
         cudaGetLastError();
 }
 
@@ -1676,7 +1691,7 @@ kf_status kf_render(kf_session* s, int mode, const float pose_in[16], uint8_t* r
     KF_CK(cudaMemsetAsync(sl.render_n, 0, size_t(w) * h * 16, st));
     const int cap = ray_queue_entries(w, h, true);
     Scratch scratch;
-    raycast_scratch(scratch, 0, cap, st);
+    raycast_scratch(scratch, 0, w, h, cap, st);
     KF_CK(stage_raycast(&vol, pose, ik, sl.render_v, sl.render_n, w, h, c.min_depth, c.max_depth, c.step_large,
                         c.step_small, scratch.p, cap, st, &bounds));
     DispMats m{};
@@ -1809,7 +1824,7 @@ kf_status kf_raycast(const kf_volume* vol, const float pose[16], const float inv
     const bool build = stage_raycast_builds_bounds(vol, w, h);
     const int cap = ray_queue_entries(w, h, build);
     Scratch scratch;
-    raycast_scratch(scratch, build ? vol->n : 0, cap, st);
+    raycast_scratch(scratch, build ? vol->n : 0, w, h, cap, st);
     StageTimer t(elapsed_ms, st);
     return t.finish(stage_raycast(vol, pose, inv_cam_k, reinterpret_cast<float4*>(vertex),
                                   reinterpret_cast<float4*>(normal), w, h, min_depth, max_depth, step_large,

@@ -23,8 +23,6 @@
 
 namespace kf {
 
-__host__ __device__ int fuse_units(int n) { return ((n + 31) / 32) * ((n + 7) / 8) * ((n + 7) / 8); }
-
 // order-preserving int key of a float (atomicMin on floats of either sign)
 __device__ __forceinline__ int fkey(float x) {
     const int i = __float_as_int(x);
@@ -336,16 +334,6 @@ template <> struct FuseLists<true> {
     static constexpr int kQueued = 8, kTaken = 9;
 };
 
-// session of global fusion unit g (binary search over the per-slot prefix)
-__device__ __forceinline__ int unit_session(const long long* prefix, long long g, int S_cap) {
-    int lo = 0, hi = S_cap;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(prefix + mid) <= g) lo = mid; else hi = mid;
-    }
-    return lo;
-}
-
 // one thread per block of every stepping session: append the blocks that can update to the
 // queue (counters[4] = entries; [8] for the visualization volumes), one atomic per warp
 template <bool kVis>
@@ -358,6 +346,14 @@ __global__ void __launch_bounds__(256, 4) fuse_cull_kernel(EngineView v) {
     const int S_cap = v.tb->S;
     const int lane = threadIdx.x & 31;
     const long long stride = (long long)gridDim.x * blockDim.x;
+    if (!kVis) {
+        // the raycast of this step is done with the sessions' depth ranges: zero for the next one
+        for (int s = blockIdx.x; s < S_cap; s += gridDim.x) {
+            const SessionDev* S = &v.sess[s];
+            if (!v.step[s].active || !S->range) continue;
+            for (int q = threadIdx.x; q < range_words(S->W, S->H); q += blockDim.x) S->range[q] = 0u;
+        }
+    }
     FuseCtx c;
     int cur_s = -1;
     bool live = false;

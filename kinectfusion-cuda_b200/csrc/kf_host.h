@@ -25,6 +25,8 @@ struct Tables {
     long long vis_fuse_total;  // the same over the slots' visualization volumes
 };
 
+constexpr int kCounters = 12;   // words of EngineView::counters
+
 struct LongRay;   // march state of a ray handed from a lane to a warp (k_raycast.cu)
 int serial_budget(int ray_tiles);   // ray_budget for a step with this many ray tiles
 bool many_ray_tiles(int ray_tiles); // a step large enough for the raycast's long-budget, 4-block form
@@ -76,6 +78,9 @@ constexpr int kIcpMaxPasses = 64;     // hard cap on ICP passes per frame
 // launch helpers (each returns the CUDA error of its launch)
 cudaError_t launch_preprocess(const EngineView& v, int grid, cudaStream_t st);
 // many: a step of more than kManyRayTiles ray tiles (serial_budget's rule)
+// The depth ranges of a step's raycast (a grid of one thread per fusion unit, or grid-stride); also
+// clears the wait record and the counters.
+cudaError_t launch_ray_range(const EngineView& v, int grid, cudaStream_t st);
 cudaError_t launch_raycast(const EngineView& v, int grid, cudaStream_t st, bool many);
 int serial_budget_many();   // the lane budget of the raycast's many-tile form
 int ray_count_slots();      // entries of the raycast's debug work counts
@@ -92,7 +97,18 @@ int icp_max_grid(int num_sms);
 int long_ray_bytes();
 cudaError_t launch_barrier_selftest(GridSync* g, unsigned long long timeout_ns, int* result, cudaStream_t st);
 cudaError_t launch_read_probe(const float4* buf, long long n4, int rounds, float* sink, int grid, cudaStream_t st);
-__host__ __device__ int fuse_units(int n);   // 32 x 8 x 8 voxel blocks of an n^3 volume
+// 32 x 8 x 8 voxel blocks of an n^3 volume
+__host__ __device__ inline int fuse_units(int n) { return ((n + 31) / 32) * ((n + 7) / 8) * ((n + 7) / 8); }
+
+// session of global fusion unit g (binary search over the per-slot prefix)
+__device__ __forceinline__ int unit_session(const long long* prefix, long long g, int S_cap) {
+    int lo = 0, hi = S_cap;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(prefix + mid) <= g) lo = mid; else hi = mid;
+    }
+    return lo;
+}
 
 cudaError_t launch_init_volume(void* f, void* w, long long nvox, int fmt, cudaStream_t st);
 cudaError_t launch_export_interleaved(const void* f, const void* w, long long nvox, int fmt, float* dst, cudaStream_t st);
@@ -109,7 +125,7 @@ cudaError_t stage_normal(const float4* v, float4* n, int w, int h, cudaStream_t 
 // size when the call builds bounds, else 0), or null to march every ray in its own thread.
 bool stage_raycast_builds_bounds(const kf_volume* vol, int w, int h);
 int stage_raycast_queue(int w, int h, bool bounds, long long share);   // share: a session's entries
-size_t stage_raycast_scratch(int n, int longq_cap);
+size_t stage_raycast_scratch(int n, int w, int h, int longq_cap);
 cudaError_t stage_raycast(const kf_volume* vol, const float* pose, const float* ik, float4* vtx, float4* nrm, int w,
                           int h, float min_d, float max_d, float step_l, float step_s, void* scratch, int longq_cap,
                           cudaStream_t st, const SessionDev* bounds = nullptr);

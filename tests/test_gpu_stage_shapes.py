@@ -79,6 +79,7 @@ def plain_raycast(kf, cuda, vol, pose, ik, v, n, step, depths):
     cuda.cuda.synchronize()
 
 
+SKEW = np.array([[1.02, 0.01, 0], [-0.02, 0.97, 0.03], [0, 0.01, 1.05]], np.float32)   # not a rotation
 VIEWS = {"loop": None, "inside": (0.1, 0.1, 0.35), "away": (3.0, 0.0, 4.0), "mirrored": None}
 
 
@@ -86,7 +87,9 @@ VIEWS = {"loop": None, "inside": (0.1, 0.1, 0.35), "away": (3.0, 0.0, 4.0), "mir
                                             (136, 500, 330, 1, "loop"), (136, 500, 330, 0, "inside"),
                                             (136, 500, 330, 0, "away"), (136, 500, 330, 0, "mirrored"),
                                             (136, 500, 331, 0, "unaligned"), (512, 640, 480, 0, "loop"),
-                                            (256, 160, 120, 1, "inside")])
+                                            (256, 160, 120, 1, "inside"), (200, 500, 330, 0, "inside"),
+                                            (200, 500, 330, 1, "away"), (200, 500, 330, 0, "mirrored"),
+                                            (264, 501, 331, 0, "loop"), (200, 500, 330, 0, "skewed")])
 def test_raycast_paths_agree(kf, orc, cuda, n, w, h, fmt, view):
     """A call with scratch (bounds from one read of the visible volume, or none; ray tiles; long
     rays by warps) gives the maps of the call without any, bit for bit: skipping and queueing
@@ -112,6 +115,8 @@ def test_raycast_paths_agree(kf, orc, cuda, n, w, h, fmt, view):
     elif view == "away":
         pose[:3, 3] = VIEWS[view]
     ik = np.linalg.inv(k.astype(np.float64)).astype(np.float32)
+    if view == "skewed":
+        pose[:3, :3] = pose[:3, :3] @ SKEW
     if view == "mirrored":
         ik = ik @ np.array([[-1, 0, w], [0, 1, 0], [0, 0, 1]], np.float32)
     out = [[cuda.full((h, w, 4), 7.0, device="cuda") for _ in range(2)] for _ in range(2)]
@@ -121,3 +126,40 @@ def test_raycast_paths_agree(kf, orc, cuda, n, w, h, fmt, view):
         assert cuda.equal(a.view(cuda.int32), b.view(cuda.int32))
     hits = float((out[0][0][..., 3] == -1).float().mean())
     assert hits > 0.05 or n == 8 or view in ("away", "inside"), hits
+
+
+@pytest.mark.parametrize("n,w,h,fmt,levels", [(192, 320, 240, 0, 3), (200, 164, 124, 1, 3), (264, 500, 330, 0, 2)])
+def test_session_depth_ranges_change_nothing(kf, cuda, n, w, h, fmt, levels):
+    """A session's raycast, whose rays start and end by their tile's depth range, equals the march
+    of every sample (plain_raycast) bit for bit at every level: at the tracked pose, at one that is
+    not exactly a rotation, looking across the volume from inside it, and looking away."""
+    from kfb200 import synth
+    cfg = kf.config_small(width=w, height=h, fx=262.5 * w / 320, fy=262.5 * w / 320, cx=w / 2 - 0.5, cy=h / 2 - 0.5,
+                          levels=levels, volume_n=n, mu=0.03, tsdf_format=fmt, keep_on_miss=0, min_depth=0.05)
+    imgs, _ = synth.sequence(cfg, 4, seed=5, kind=synth.LOOP)
+    s = kf.KinectFusion(cfg)
+    for img in imgs[:3]:
+        s.process_frame(img)
+    tracked = s.pose()
+    poses = [tracked, tracked.copy(), tracked.copy(), tracked.copy()]
+    poses[1][:3, :3] = poses[1][:3, :3] @ SKEW
+    poses[2][:3, 3] = (0.1, 0.1, 0.0)
+    poses[2][:3, :3] = np.array([[0, 0, 1], [0, 1, 0], [-1, 0, 0]], np.float32)
+    poses[3][:3, 3] = (3.0, 0.0, 4.0)
+    for pose in poses:
+        f, wt = s.tsdf()
+        ft = cuda.from_numpy(f).cuda()
+        ft = ft.half() if fmt else ft
+        vol = kf.kernel.volume(ft, cuda.zeros_like(ft), cfg.volume_width, cfg.mu, fmt=fmt)
+        s.set_pose(pose)
+        s.process_frame(imgs[3])
+        for level in range(levels):
+            wl, hl = w >> level, h >> level
+            want = [cuda.zeros((hl, wl, 4), device="cuda") for _ in range(2)]
+            for m in want:
+                m[..., 3] = -2
+            plain_raycast(kf, cuda, vol, pose, kf.level_inverse_intrinsics(cfg, level), *want,
+                          (cfg.step_large, cfg.step_small), (cfg.min_depth, cfg.max_depth))
+            for a, b in zip(s.raycast_maps(level), want):
+                np.testing.assert_array_equal(a.view(np.int32), b.cpu().numpy().view(np.int32))
+    s.close()
