@@ -121,7 +121,7 @@ void pose16_to_double(const float* p, double* R, double* t) {
     for (int r = 0; r < 3; ++r) t[r] = p[12 + r];
 }
 
-// initial device pose state: estimate = previous = pose, float mirrors, inverse
+// initial device pose state: estimate = previous = pose, float mirrors
 PoseDev make_pose_dev(const float* pose16) {
     PoseDev P;
     std::memset(&P, 0, sizeof(P));
@@ -130,12 +130,7 @@ PoseDev make_pose_dev(const float* pose16) {
     std::memcpy(P.t, P.tp, sizeof(P.t));
     for (int q = 0; q < 9; ++q) P.Rpf[q] = float(P.Rp[q]);
     for (int q = 0; q < 3; ++q) P.tpf[q] = float(P.tp[q]);
-    for (int c = 0; c < 3; ++c)
-        for (int r = 0; r < 3; ++r) P.iRf[c * 3 + r] = float(P.Rp[r * 3 + c]);
-    for (int r = 0; r < 3; ++r)
-        P.itf[r] = float(-(P.Rp[r * 3 + 0] * P.tp[0] + P.Rp[r * 3 + 1] * P.tp[1] + P.Rp[r * 3 + 2] * P.tp[2]));
     P.level = -1;
-    P.fuse_ok = 1;
     return P;
 }
 
@@ -455,7 +450,7 @@ struct Shape {
     int ray_budget = 0;   // 0: by the ray-tile count (serial_budget); else march iterations a lane
                           // takes before queueing its ray for a warp
     int ray_tw = kRayTileW;   // ray tile width (32 / ray_tw rows)
-    int fuse_split = 0;   // 0: by the queue length (fuse_split); 1, 2, 4: entries whole, halves, quarters
+    int fuse_split = 0;   // 0: by the queue length (fuse_split()); 1, 2, 4: as many warps share a half unit
     bool operator==(const Shape& o) const {
         return grid_pre == o.grid_pre && grid_ray == o.grid_ray && grid_fuse == o.grid_fuse &&
                grid_icp == o.grid_icp && ray_form == o.ray_form &&
@@ -500,6 +495,7 @@ struct Engine {
     std::vector<Slot> slots;
     // device
     SessionDev* d_sess = nullptr;
+    FuseCtx* d_fctx = nullptr;   // 2 x cap: the tracking volumes' fusion contexts, the visualization volumes'
     StepDev* d_step = nullptr;
     OutDev* d_out = nullptr;
     Tables* d_tb = nullptr;
@@ -521,12 +517,13 @@ struct Engine {
     // long-ray queue of the raycaster (bytes; entries = bytes / long_ray_bytes())
     char* d_longq = nullptr;
     int cap_longq = 0;
-    // fusion queue (one entry per block of every slot at most), and the visualization volumes'
-    unsigned int* d_fuseq = nullptr;
+    // fusion queue (one entry per half unit of every slot at most), and the visualization volumes'
+    uint2* d_fuseq = nullptr;
     int cap_fuseq = 0;
-    unsigned int* d_vfuseq = nullptr;
+    uint2* d_vfuseq = nullptr;
     int cap_vfuseq = 0;
     bool has_vis = false;      // some slot has a visualization volume: the step fuses it too
+    int fuse_fmt = -1;         // the volume format of every slot, or -1: slots of both
     bool has_range = false;    // some slot's raycast takes depth ranges: the step makes them
     unsigned long long* d_ray_counts = nullptr;   // debug mode KF_DEBUG_COUNTERS: raycast work counts
     bool count_rays = false;
@@ -572,6 +569,8 @@ struct Engine {
         KF_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         KF_CK(cudaMalloc(&d_sess, sizeof(SessionDev) * capacity));
         KF_CK(cudaMemset(d_sess, 0, sizeof(SessionDev) * capacity));
+        KF_CK(cudaMalloc(&d_fctx, 2 * sizeof(FuseCtx) * capacity));
+        KF_CK(cudaMemset(d_fctx, 0, 2 * sizeof(FuseCtx) * capacity));
         KF_CK(cudaMalloc(&d_step, sizeof(StepDev) * capacity));
         KF_CK(cudaMemset(d_step, 0, sizeof(StepDev) * capacity));
         static_assert(sizeof(OutDev) % 16 == 0 && sizeof(GridSync) % 16 == 0, "result block layout");
@@ -660,7 +659,7 @@ struct Engine {
         for (Slot& s : slots) if (!s.external) s.release();
         for (cudaEvent_t& e : ev)
             if (e) cudaEventDestroy(e);
-        cudaFree(d_sess); cudaFree(d_step); cudaFree(d_out); cudaFree(d_tb); cudaFree(d_pre); cudaFree(d_ray);
+        cudaFree(d_sess); cudaFree(d_fctx); cudaFree(d_step); cudaFree(d_out); cudaFree(d_tb); cudaFree(d_pre); cudaFree(d_ray);
         cudaFree(d_itiles); cudaFree(d_iranges); cudaFree(d_fprefix);
         cudaFree(d_vfprefix); cudaFree(d_vfuseq);
         cudaFree(d_ray_counts);
@@ -681,7 +680,7 @@ struct Engine {
 
     EngineView view() const {
         EngineView v;
-        v.sess = d_sess; v.step = d_step; v.out = d_out; v.tb = d_tb; v.pre = d_pre; v.ray = d_ray;
+        v.sess = d_sess; v.fctx = d_fctx; v.vis_fctx = d_fctx + cap; v.step = d_step; v.out = d_out; v.tb = d_tb; v.pre = d_pre; v.ray = d_ray;
         v.itiles = d_itiles; v.iranges = d_iranges; v.fuse_prefix = d_fprefix;
         v.partials = d_partials;
         v.partials2 = d_partials ? d_partials + cap_part / 2 : nullptr;   // two equal halves
@@ -724,10 +723,10 @@ struct Engine {
         long long cur_it = 0;
         for (int l = 0; l < KF_MAX_LEVELS; ++l) cur_it += tb.n_itiles[l];
         const long long need_it = cur_it + res_it;
-        const long long need_fq = tb.fuse_total + res_fq;
-        const long long need_vfq = tb.vis_fuse_total + res_vfq;
+        const long long need_fq = 2 * (tb.fuse_total + res_fq);   // two halves per unit
+        const long long need_vfq = 2 * (tb.vis_fuse_total + res_vfq);
         if (need_pre > INT32_MAX || long_ray_entries(need_ray * 32) > INT32_MAX / long_ray_bytes() ||
-            need_it * kIcpPartialStride > INT32_MAX || need_fq > (1 << 29) || need_vfq > (1 << 29))
+            need_it * kIcpPartialStride > INT32_MAX || need_fq > INT32_MAX || need_vfq > INT32_MAX)
             return KF_ERR_CAPACITY;
         const int old_pre = cap_pre, old_ray = cap_ray, old_it = cap_it, old_part = cap_part, old_lq = cap_longq,
                   old_fq = cap_fuseq;
@@ -755,17 +754,22 @@ struct Engine {
         std::vector<IcpRange> ranges(size_t(KF_MAX_LEVELS) * cap, IcpRange{0, 0});
         std::vector<long long> fprefix(cap + 1, 0), vfprefix(cap + 1, 0);
         std::vector<SessionDev> sess(cap);
+        std::vector<FuseCtx> fctx(2 * cap, FuseCtx{});
         int max_levels = 1;
         bool range = false;
+        int formats = 0;
         for (int s = 0; s < cap; ++s) {
             const Slot& sl = slots[s];
             fprefix[s + 1] = fprefix[s];
             vfprefix[s + 1] = vfprefix[s];
             if (!sl.used) { std::memset(&sess[s], 0, sizeof(SessionDev)); continue; }
             sess[s] = sl.d;
+            fctx[s] = fuse_context(sl.d, false);
+            fctx[cap + s] = fuse_context(sl.d, true);
             const kf_config& c = sl.cfg;
             max_levels = std::max(max_levels, c.levels);
             range |= sl.d.range != nullptr;
+            formats |= 1 << sl.d.fmt;
             if (!sl.external) {
                 for (int y = 0; y < c.height; y += kPreTileSize)
                     for (int x = 0; x < c.width; x += kPreTileSize) pre.push_back(PreTile{s, x, y});
@@ -810,15 +814,18 @@ struct Engine {
         }
         const int old_pre = cap_pre, old_ray = cap_ray, old_it = cap_it, old_part = cap_part, old_lq = cap_longq,
                   old_fq = cap_fuseq;
-        // fusion queue entries are 32-bit and each is taken in 4 parts counted in 32 bits
+        // two fusion queue entries per unit; their items (quarters of entries) are counted in 32 bits
         if (fprefix[cap] > (long long)(1 << 29) || vfprefix[cap] > (long long)(1 << 29)) return KF_ERR_CAPACITY;
-        KF_TRY(grow(d_fuseq, cap_fuseq, std::max<int>(1, int(fprefix[cap]))));
+        KF_TRY(grow(d_fuseq, cap_fuseq, std::max<int>(1, int(2 * fprefix[cap]))));
         const int old_vfq = cap_vfuseq;
-        KF_TRY(grow(d_vfuseq, cap_vfuseq, std::max<int>(1, int(vfprefix[cap]))));
+        KF_TRY(grow(d_vfuseq, cap_vfuseq, std::max<int>(1, int(2 * vfprefix[cap]))));
         if (old_vfq != cap_vfuseq) graph_dirty = true;
         const bool vis = vfprefix[cap] > 0;
         if (vis != has_vis) graph_dirty = true;   // the step launches the visualization fusion or not
         has_vis = vis;
+        const int fmt = formats == 1 << KF_TSDF_F32F32 ? KF_TSDF_F32F32 : formats == 1 << KF_TSDF_F16U16 ? KF_TSDF_F16U16 : -1;
+        if (fmt != fuse_fmt) graph_dirty = true;   // the step's fusion kernel is built for the format
+        fuse_fmt = fmt;
         if (range != has_range) graph_dirty = true;   // the step makes depth ranges or not
         has_range = range;
         KF_TRY(grow(d_pre, cap_pre, std::max<int>(1, int(pre.size()))));
@@ -837,6 +844,7 @@ struct Engine {
         KF_CK(cudaMemcpy(d_fprefix, fprefix.data(), sizeof(long long) * fprefix.size(), cudaMemcpyHostToDevice));
         KF_CK(cudaMemcpy(d_vfprefix, vfprefix.data(), sizeof(long long) * vfprefix.size(), cudaMemcpyHostToDevice));
         KF_CK(cudaMemcpy(d_sess, sess.data(), sizeof(SessionDev) * cap, cudaMemcpyHostToDevice));
+        KF_CK(cudaMemcpy(d_fctx, fctx.data(), sizeof(FuseCtx) * 2 * cap, cudaMemcpyHostToDevice));
         tb.S = cap;
         tb.n_pre = int(pre.size());
         tb.n_ray = int(ray.size());
@@ -899,13 +907,13 @@ struct Engine {
         if (profile) KF_CK(cudaEventRecordWithFlags(ev[3], st, cudaEventRecordExternal));
         {
             NvtxRange r("kf.fusion");
-            if (stages[3]) KF_CK(launch_fuse(v, shape.grid_fuse, st));
+            if (stages[3]) KF_CK(launch_fuse(v, shape.grid_fuse, fuse_fmt, st));
         }
         if (has_vis && stages[3]) {
             // the visualization volumes (the reference's second grid), after the tracking fusion
             // and in the same stage time
             NvtxRange r("kf.fusion_vis");
-            KF_CK(launch_fuse_vis(v, shape.grid_fuse, st));
+            KF_CK(launch_fuse_vis(v, shape.grid_fuse, fuse_fmt, st));
         }
         if (profile) KF_CK(cudaEventRecordWithFlags(ev[4], st, cudaEventRecordExternal));
         return KF_OK;

@@ -535,7 +535,7 @@ __device__ void icp_solve(const EngineView& v, int s, int level, int begin, int 
 
 // phase C for one session (one thread): the frame's pose becomes the previous pose; the
 // inverse feeds fusion; the result block goes to the host.
-__device__ void icp_finish(const SessionDev* S, const StepDev st, OutDev* out) {
+__device__ void icp_finish(const SessionDev* S, const StepDev st, OutDev* out, FuseCtx* fctx, FuseCtx* vis_fctx) {
     if (!st.active) return;
     PoseDev* P = S->pose;
     const bool ok = P->status == KF_OK;
@@ -545,12 +545,17 @@ __device__ void icp_finish(const SessionDev* S, const StepDev st, OutDev* out) {
     }
     for (int q = 0; q < 9; ++q) P->Rpf[q] = float(P->Rp[q]);
     for (int q = 0; q < 3; ++q) P->tpf[q] = float(P->tp[q]);
-    // inverse: R^T, -R^T t
+    // inverse, for the frame's fusion: R^T, -R^T t
+    float iR[9], it[3];
     for (int c = 0; c < 3; ++c)
-        for (int r = 0; r < 3; ++r) P->iRf[c * 3 + r] = float(P->Rp[r * 3 + c]);
+        for (int r = 0; r < 3; ++r) iR[c * 3 + r] = float(P->Rp[r * 3 + c]);
     for (int r = 0; r < 3; ++r)
-        P->itf[r] = float(-(P->Rp[r * 3 + 0] * P->tp[0] + P->Rp[r * 3 + 1] * P->tp[1] + P->Rp[r * 3 + 2] * P->tp[2]));
-    P->fuse_ok = ok ? 1 : 0;
+        it[r] = float(-(P->Rp[r * 3 + 0] * P->tp[0] + P->Rp[r * 3 + 1] * P->tp[1] + P->Rp[r * 3 + 2] * P->tp[2]));
+    for (FuseCtx* f : {fctx, vis_fctx}) {
+        for (int q = 0; q < 9; ++q) f->iR[q] = iR[q];
+        for (int q = 0; q < 3; ++q) f->it[q] = it[q];
+        f->ok = ok ? 1 : 0;
+    }
     P->frame += 1;
     for (int q = 0; q < 16; ++q) out->pose[q] = 0.f;
     for (int c = 0; c < 3; ++c)
@@ -726,11 +731,11 @@ __global__ void __launch_bounds__(kIcpThreads, local ? 1 : 2) icp_kernel(EngineV
         // block 0 stores the state the rest of the frame and the host read
         if (blockIdx.x == 0 && tid == 0 && v.step[0].active) {
             store_local_state(v.sess[0].pose, loc, v.step[0].first != 0);
-            icp_finish(&v.sess[0], v.step[0], v.out);
+            icp_finish(&v.sess[0], v.step[0], v.out, v.fctx, v.vis_fctx);
         }
     } else {
         for (int s = blockIdx.x; s < S_cap; s += gridDim.x)
-            if (tid == 0) icp_finish(&v.sess[s], v.step[s], v.out + s);
+            if (tid == 0) icp_finish(&v.sess[s], v.step[s], v.out + s, v.fctx + s, v.vis_fctx + s);
     }
 }
 

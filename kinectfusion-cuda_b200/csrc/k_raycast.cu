@@ -158,7 +158,7 @@ __device__ __forceinline__ unsigned int range_candidates(int n, int nb, const in
     const int ux = (n + 31) >> 5, uy = n >> 3;
     const int bx = (u % ux) * 4, byz = u / ux, by = byz % uy, bz = byz / uy;
     const int* b = bdil + (bz * nb + by) * nb + bx;
-    const int thr = __float_as_int(0.991f);
+    const int thr = __float_as_int(kSkipLarge);
     if ((nb & 3) == 0) {   // rows of bounds start on 16 bytes
         const int4 k = __ldg(reinterpret_cast<const int4*>(b));
         return (k.x < thr ? 1u : 0u) | (k.y < thr ? 2u : 0u) | (k.z < thr ? 4u : 0u) | (k.w < thr ? 8u : 0u);
@@ -168,29 +168,6 @@ __device__ __forceinline__ unsigned int range_candidates(int n, int nb, const in
     for (int q = 0; q < 4; ++q)
         if (bx + q < nb && __ldg(b + q) < thr) m |= 1u << q;
     return m;
-}
-
-// The candidates of a block's 256 units, packed into list as (thread << 2 | brick): a surface's bricks
-// lie in few warps' units (a floor crosses all of a row's), so the block shares them out.  Returns how
-// many; every thread of the block calls it.
-__device__ __forceinline__ int range_pack(unsigned int m, unsigned short* list, int* count) {
-    const int lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) *count = 0;
-    __syncthreads();
-    if (__any_sync(0xffffffffu, m != 0)) {
-        int incl = __popc(m);
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, off);
-            if (lane >= off) incl += y;
-        }
-        int at = 0;
-        if (lane == 31) at = atomicAdd(count, incl);
-        at = __shfl_sync(0xffffffffu, at, 31) + incl - __popc(m);
-        for (; m; m &= m - 1) list[at++] = (unsigned short)((threadIdx.x << 2) | (__ffs(m) - 1));
-    }
-    __syncthreads();
-    return *count;
 }
 
 // march state: everything the reference's loop carries from one sample to the next
@@ -456,7 +433,7 @@ __device__ __forceinline__ bool skip_cell(const SessionDev* S, const RayGeo& g, 
                                           float inc) {
     const int n = S->n;
     // order-preserving int keys of the two thresholds
-    const int thr = st.small ? __float_as_int(0.001f) : __float_as_int(0.991f);
+    const int thr = st.small ? __float_as_int(kSkipSmall) : __float_as_int(kSkipLarge);
     const int sx = vx >> 5, sy = vy >> 5, sz = vz >> 5;
     const int ns = S->ns, nb = S->nb;   // (n / 8)^3 bricks: 32-bit indices
     float exit_t;
@@ -807,7 +784,7 @@ __global__ void __launch_bounds__(256) ray_range_kernel(EngineView v) {
             if (st.active && !st.first && S->range)
                 m = range_candidates(S->n, S->nb, S->bdil, int(base + tid - __ldg(v.fuse_prefix + s)));
         }
-        const int count = range_pack(m, list, &packed);
+        const int count = block_pack(m, list, &packed);
         for (int i = tid & ~31; i < count; i += 256) {
             bool on = i + (tid & 31) < count;
             int bx = 0, by = 0, bz = 0;
@@ -1075,7 +1052,7 @@ __global__ void __launch_bounds__(256) range_stage_kernel(const __grid_constant_
     __shared__ unsigned short list[256 * 4];
     __shared__ int packed;
     const int tid = threadIdx.x, u0 = blockIdx.x * blockDim.x, ux = (r.n + 31) >> 5;
-    const int count = range_pack(u0 + tid < fuse_units(r.n) ? range_candidates(r.n, r.nb, bdil, u0 + tid) : 0u, list, &packed);
+    const int count = block_pack(u0 + tid < fuse_units(r.n) ? range_candidates(r.n, r.nb, bdil, u0 + tid) : 0u, list, &packed);
     for (int i = tid & ~31; i < count; i += 256) {
         const bool on = i + (tid & 31) < count;
         const int code = on ? list[i + (tid & 31)] : 0, u = u0 + (code >> 2);

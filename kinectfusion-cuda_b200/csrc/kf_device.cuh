@@ -16,6 +16,9 @@ constexpr float kValid = -1.0f;     // project/src/device_helper.cuh:9
 constexpr float kInvalid = -2.0f;   // project/src/device_helper.cuh:10
 constexpr float kMinDepth = 0.01f;  // project/src/device_helper.cuh:11
 constexpr int kMaxBilateralRadius = 7;
+// A sample at or above kSkipLarge cannot change the raycast's large steps, one at or above kSkipSmall
+// cannot change its small steps (its tests are below 0.99 and below 0, with a margin for rounding).
+constexpr float kSkipLarge = 0.991f, kSkipSmall = 0.001f;
 constexpr int kRangeTile = 16;      // pixels per side of a depth-range tile of the raycast
 // Volumes from this size on get depth ranges (k_raycast.cu).  They cost a launch of about 5 us; the
 // skips they save grow with n.  One frame: 512x424 in 256^3 201 us with, 210 without; 320x240 in
@@ -41,14 +44,12 @@ struct PoseDev {
     double R[9], t[3];      // ICP estimate, camera->world, column-major R
     double Rp[9], tp[3];    // pose of the previous frame
     float Rpf[9], tpf[3];   // float copy of the previous pose (raycast, correspondence)
-    float iRf[9], itf[3];   // inverse of the frame's final pose (world->camera) for fusion
     int iters[kMaxLevels];  // ICP iterations run per level in the current frame
     int level;              // level of the next ICP pass (-1 once ICP is finished)
     int it;                 // iteration index within that level
     int cont;               // 1 while this session takes part in the next ICP pass
     int status;             // kf_status of the current frame
     int frame;              // frames processed so far
-    int fuse_ok;            // 1 when this frame's fusion runs
 };
 
 // a session's visualization volume (n = 0: none): a second TSDF in the session's format, fused
@@ -113,6 +114,27 @@ struct SessionDev {
     float angle_cos;       // cos(angle_th): the normal test compares cosines
     PoseDev* pose;
     VisDev vis;
+};
+
+// everything fusion needs about one volume of one session, as one block that a warp or a thread reads
+// at once: the constants written by the host, the pose by the ICP kernel at the end of every frame
+struct __align__(16) FuseCtx {
+    float iR[9], it[3];          // world -> camera of the frame being fused
+    float fx, fy, cx, cy;
+    float min_d, max_d, mu, max_w;
+    const float* depth;          // unfiltered metres map
+    const float* dmax;           // per 16x16 tile: largest valid depth
+    int t16w, ok;                // tiles per row; 1 when this frame's fusion runs
+    int w, h;
+    int n, nb, ns, fmt;
+    void* F;
+    void* W;
+    const float* xs;
+    const float* zs;
+    int* bmin;                   // brick lower bounds (null: none kept)
+    int* bdil;                   // their widenings to the bricks and super-bricks around them
+    int* sdil;
+    void* pad;
 };
 
 // per-step control, written by the host: which sessions take part and which are on their

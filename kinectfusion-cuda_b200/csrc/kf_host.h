@@ -19,8 +19,8 @@ struct Tables {
     int max_levels;
     int ray_budget;          // march iterations a lane takes before handing its ray to a warp
     int ray_tw;              // ray tile width (a warp's 32 rays are ray_tw x 32 / ray_tw pixels)
-    int fuse_split;          // 0: fusion takes queue entries by the rule of fuse_split(); 1, 2, 4:
-                             // whole, in halves or in quarters
+    int fuse_split;          // 0: fusion warps share a half unit by the rule of fuse_split(); 1, 2, 4:
+                             // as many warps per half unit
     long long fuse_total;    // fusion segments over all slots
     long long vis_fuse_total;  // the same over the slots' visualization volumes
 };
@@ -30,6 +30,30 @@ constexpr int kCounters = 12;   // words of EngineView::counters
 struct LongRay;   // march state of a ray handed from a lane to a warp (k_raycast.cu)
 int serial_budget(int ray_tiles);   // ray_budget for a step with this many ray tiles
 bool many_ray_tiles(int ray_tiles); // a step large enough for the raycast's long-budget, 4-block form
+
+// The candidates of a block's 256 fusion units, packed into list (1024 entries) as
+// (thread << 2 | brick), m the calling thread's brick mask: a surface's blocks lie in few warps'
+// units (a floor crosses all of a row's), so the block shares them out.  Returns how many; every
+// thread of the block calls it.
+__device__ __forceinline__ int block_pack(unsigned int m, unsigned short* list, int* count) {
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) *count = 0;
+    __syncthreads();
+    if (__any_sync(0xffffffffu, m != 0)) {
+        int incl = __popc(m);
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += y;
+        }
+        int at = 0;
+        if (lane == 31) at = atomicAdd(count, incl);
+        at = __shfl_sync(0xffffffffu, at, 31) + incl - __popc(m);
+        for (; m; m &= m - 1) list[at++] = (unsigned short)((threadIdx.x << 2) | (__ffs(m) - 1));
+    }
+    __syncthreads();
+    return *count;
+}
 
 // raw pointers the kernels take
 struct EngineView {
@@ -41,6 +65,8 @@ struct EngineView {
     const RayTile* ray;
     const IcpTile* itiles;
     const IcpRange* iranges;     // [level * S + s]
+    FuseCtx* fctx;               // per slot: the tracking volume's fusion context
+    FuseCtx* vis_fctx;           // the visualization volume's
     const long long* fuse_prefix;// S + 1 entries, in segments
     const long long* vis_fuse_prefix;   // the same for the visualization volumes
     float* partials;             // ICP tile partials, kIcpPartialStride floats per tile
@@ -48,14 +74,14 @@ struct EngineView {
     int4* icp_sched;             // per slot: {level of the next ICP pass or -1, first tile, tiles, 0}
     float* icp_mats;             // per slot: 24 floats phase A reads (R, t, K_l R_prev^T, t_prev)
     GridSync* sync;
-    unsigned int* counters;      // [0] raycast tiles, [4] fusion blocks queued, [5] fusion
-                                 // items taken, [6] long rays queued, [7] long rays taken,
-                                 // [8], [9] the visualization volumes' [4], [5]
+    unsigned int* counters;      // [0] raycast tiles, [4] fusion half units queued, [5] fusion items
+                                 // taken, [6] long rays queued, [7] long rays taken, [8], [9] the
+                                 // visualization volumes' [4], [5]
     LongRay* longq;              // long-ray queue
     int longq_cap;
-    unsigned int* fuseq;         // fusion queue: global unit index of each block that can update
+    uint2* fuseq;                // fusion queue: {slot, first brick} of each half unit that can update
     int fuseq_cap;
-    unsigned int* vis_fuseq;     // the visualization volumes' fusion queue
+    uint2* vis_fuseq;     // the visualization volumes' fusion queue
     int vis_fuseq_cap;
     unsigned long long* ray_counts;   // debug mode: the raycast's work counts (null: not counted)
 };
@@ -86,9 +112,12 @@ int serial_budget_many();   // the lane budget of the raycast's many-tile form
 int ray_count_slots();      // entries of the raycast's debug work counts
 // single: an engine of one slot (the kernel keeps that session's state per block)
 cudaError_t launch_icp(const EngineView& v, int grid, cudaStream_t st, bool single);
-cudaError_t launch_fuse(const EngineView& v, int grid, cudaStream_t st);
+// fmt: the volume format every slot has, or -1 for slots of both
+cudaError_t launch_fuse(const EngineView& v, int grid, int fmt, cudaStream_t st);
+// the constant part of a session's fusion context (its tracking or its visualization volume)
+FuseCtx fuse_context(const SessionDev& d, bool vis);
 // the same for the sessions' visualization volumes (cull, fuse and bounds)
-cudaError_t launch_fuse_vis(const EngineView& v, int grid, cudaStream_t st);
+cudaError_t launch_fuse_vis(const EngineView& v, int grid, int fmt, cudaStream_t st);
 // bounds = key(2), the initial distance; rebuild recomputes them exactly from a loaded volume
 cudaError_t launch_init_bricks(int* bmin, int* bdil, int* sdil, int n, cudaStream_t st);
 cudaError_t launch_widen_bricks(const int* bmin, int* bdil, int* sdil, int n, cudaStream_t st);
