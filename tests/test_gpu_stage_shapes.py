@@ -163,3 +163,35 @@ def test_session_depth_ranges_change_nothing(kf, cuda, n, w, h, fmt, levels):
             for a, b in zip(s.raycast_maps(level), want):
                 np.testing.assert_array_equal(a.view(np.int32), b.cpu().numpy().view(np.int32))
     s.close()
+
+
+@pytest.mark.parametrize("sizes", [(8, 40, 72), (136, 24, 200)])
+def test_session_fusion_equals_the_stage(kf, cuda, sizes):
+    """The first frame of sessions of both formats stepped together, alone and through kf_fuse on the
+    same depth map, at a pose without rotation (so the three form the same world-to-camera floats):
+    the same volumes bit for bit, in sizes that no unit of fusion divides."""
+    from kfb200 import synth
+    cfgs = [kf.config_small(width=164, height=124, fx=134.0, fy=134.0, cx=81.5, cy=61.5, volume_n=n,
+                            mu=max(0.03, 3.0 / n), tsdf_format=i % 2) for i, n in enumerate(sizes)]
+    imgs = [synth.sequence(c, 1, seed=3 + i)[0][0] for i, c in enumerate(cfgs)]
+    b = kf.Batch(cfgs)
+    b.step(imgs)
+    for i, (c, img) in enumerate(zip(cfgs, imgs)):
+        alone = kf.KinectFusion(c)
+        alone.process_frame(img)
+        n = c.volume_n
+        f = cuda.empty((n, n, n), dtype=cuda.float16 if c.tsdf_format else cuda.float32, device="cuda")
+        wt = cuda.empty((n, n, n), dtype=cuda.int16 if c.tsdf_format else cuda.float32, device="cuda")
+        vol = kf.kernel.volume(f, wt, c.volume_width, c.mu, fmt=c.tsdf_format)
+        kf.kernel.initializeGrid(vol)
+        pose = np.array(list(c.initial_pose), np.float32).reshape(4, 4).T
+        kf.kernel.fuse(dev(cuda, alone.depth(-1)), vol, pose, kf.level_intrinsics(c, 0))
+        w = wt.cpu().numpy()
+        w = w.view(np.uint16).astype(np.float32) / np.float32(kf.KF_WEIGHT_SCALE) if c.tsdf_format else w
+        for s in (alone, b.session(i)):
+            sf, sw = s.tsdf()
+            np.testing.assert_array_equal(sf, f.float().cpu().numpy())
+            np.testing.assert_array_equal(sw, w)
+        assert n == 8 or (w > 0).any()
+        alone.close()
+    b.close()
