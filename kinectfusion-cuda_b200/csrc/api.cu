@@ -523,7 +523,7 @@ struct Engine {
     uint2* d_vfuseq = nullptr;
     int cap_vfuseq = 0;
     bool has_vis = false;      // some slot has a visualization volume: the step fuses it too
-    int fuse_fmt = -1;         // the volume format of every slot, or -1: slots of both
+    int slot_fmt = kAnyFormat;   // the volume format every slot has, or kAnyFormat: slots of both
     bool has_range = false;    // some slot's raycast takes depth ranges: the step makes them
     unsigned long long* d_ray_counts = nullptr;   // debug mode KF_DEBUG_COUNTERS: raycast work counts
     bool count_rays = false;
@@ -823,9 +823,9 @@ struct Engine {
         const bool vis = vfprefix[cap] > 0;
         if (vis != has_vis) graph_dirty = true;   // the step launches the visualization fusion or not
         has_vis = vis;
-        const int fmt = formats == 1 << KF_TSDF_F32F32 ? KF_TSDF_F32F32 : formats == 1 << KF_TSDF_F16U16 ? KF_TSDF_F16U16 : -1;
-        if (fmt != fuse_fmt) graph_dirty = true;   // the step's fusion kernel is built for the format
-        fuse_fmt = fmt;
+        const int fmt = formats == 1 << KF_TSDF_F32F32 ? KF_TSDF_F32F32 : formats == 1 << KF_TSDF_F16U16 ? KF_TSDF_F16U16 : kAnyFormat;
+        if (fmt != slot_fmt) graph_dirty = true;   // the step's kernels are built for the format
+        slot_fmt = fmt;
         if (range != has_range) graph_dirty = true;   // the step makes depth ranges or not
         has_range = range;
         KF_TRY(grow(d_pre, cap_pre, std::max<int>(1, int(pre.size()))));
@@ -896,7 +896,7 @@ struct Engine {
         }
         {
             NvtxRange r("kf.raycast");
-            if (stages[1]) KF_CK(launch_raycast(v, shape.grid_ray, st, ray_many));
+            if (stages[1]) KF_CK(launch_raycast(v, shape.grid_ray, slot_fmt, st, ray_many));
         }
         if (fork) KF_CK(cudaStreamWaitEvent(st, ev_join, 0));
         if (profile) KF_CK(cudaEventRecordWithFlags(ev[2], st, cudaEventRecordExternal));
@@ -907,13 +907,13 @@ struct Engine {
         if (profile) KF_CK(cudaEventRecordWithFlags(ev[3], st, cudaEventRecordExternal));
         {
             NvtxRange r("kf.fusion");
-            if (stages[3]) KF_CK(launch_fuse(v, shape.grid_fuse, fuse_fmt, st));
+            if (stages[3]) KF_CK(launch_fuse(v, shape.grid_fuse, slot_fmt, st));
         }
         if (has_vis && stages[3]) {
             // the visualization volumes (the reference's second grid), after the tracking fusion
             // and in the same stage time
             NvtxRange r("kf.fusion_vis");
-            KF_CK(launch_fuse_vis(v, shape.grid_fuse, fuse_fmt, st));
+            KF_CK(launch_fuse_vis(v, shape.grid_fuse, slot_fmt, st));
         }
         if (profile) KF_CK(cudaEventRecordWithFlags(ev[4], st, cudaEventRecordExternal));
         return KF_OK;

@@ -284,10 +284,22 @@ __device__ __forceinline__ void texel(const RayGeo& g, float t, float& x, float&
     z = __fmaf_rn(__fmaf_rn(g.dir.z, t, g.o.z), g.sc, g.off);
 }
 
+__device__ __forceinline__ void clamp_voxel(int n, int& x, int& y, int& z) {
+    x = min(max(x, 0), n - 1);
+    y = min(max(y, 0), n - 1);
+    z = min(max(z, 0), n - 1);
+}
+
+__device__ __forceinline__ unsigned int voxel_index(unsigned int n, int x, int y, int z) {
+    return (unsigned(z) * n + unsigned(y)) * n + unsigned(x);
+}
+
 template <class TF>
 __device__ __forceinline__ float sample_at(const SessionDev* S, const RayGeo& g, const TF* f, float t) {
     float x, y, z;
     texel(g, t, x, y, z);
+    const InnerBase b = inner_base(S->n, x, y, z);
+    if (b.in) return trilinear_inner(f, unsigned(S->n), voxel_index(unsigned(S->n), b.x0, b.y0, b.z0), b.ax, b.ay, b.az);
     return trilinear(f, S->n, x, y, z);
 }
 
@@ -423,39 +435,26 @@ __device__ __forceinline__ void skip_to(RayState& st, float lim, float inc) {
 // march.  If the sample at st.t, with base voxel (vx, vy, vz), is such a sample, advance st past
 // every following sample in the same cell -- the run of skippable 32^3 super-bricks along the
 // ray when its super-brick qualifies, else its 8^3 brick -- to the first sample index whose
-// position is at or past the cell's (run's) exit, and return true.  kEager issues the brick
-// bound's load beside the super-brick bound's (an evaluated sample needs both): one L1/L2 round
-// trip instead of two where latency bounds the march (a single session's raycast, the long
-// rays: +0.9 % for one session); where instruction issue bounds it (the 64-register form for
-// many ray tiles) the load after a failed super-brick test only is cheaper (0.8 %).
+// position is at or past the cell's (run's) exit, and return true.  The brick's bound decides (a
+// super-brick's is the minimum over its bricks', so a skippable super-brick has no other).  The
+// super-brick's is read by a skip only, since with the depth ranges most iterations evaluate their
+// sample; kEager reads it beside the brick's, in one round trip, where latency bounds the march (a
+// single session: 38 us against 42 for 320x240 in 128^3).  With the taps' and the gradient's shared
+// arithmetic and a kernel per volume format the raycast of 24 full-size sessions went from 785 to
+// 671 us.
 template <bool kEager>
 __device__ __forceinline__ bool skip_cell(const SessionDev* S, const RayGeo& g, RayState& st, int vx, int vy, int vz,
                                           float inc) {
-    const int n = S->n;
     // order-preserving int keys of the two thresholds
     const int thr = st.small ? __float_as_int(kSkipSmall) : __float_as_int(kSkipLarge);
-    const int sx = vx >> 5, sy = vy >> 5, sz = vz >> 5;
-    const int ns = S->ns, nb = S->nb;   // (n / 8)^3 bricks: 32-bit indices
-    float exit_t;
-    if constexpr (kEager) {
-        const int bx = vx >> 3, by = vy >> 3, bz = vz >> 3;
-        const int skey = ld_keep(S->sdil + (sz * ns + sy) * ns + sx);
-        const int bkey = ld_keep(S->bdil + (bz * nb + by) * nb + bx);
-        if (skey >= thr) {
-            exit_t = superbrick_run_exit(S, g, thr, sx, sy, sz, st.far_d);
-        } else {
-            if (bkey < thr) return false;
-            exit_t = box_exit(g, n, bx * 8, bx * 8 + 8, by * 8, by * 8 + 8, bz * 8, bz * 8 + 8, st.far_d);
-        }
-    } else {
-        if (__ldg(S->sdil + (sz * ns + sy) * ns + sx) >= thr) {
-            exit_t = superbrick_run_exit(S, g, thr, sx, sy, sz, st.far_d);
-        } else {
-            const int bx = vx >> 3, by = vy >> 3, bz = vz >> 3;
-            if (__ldg(S->bdil + (bz * nb + by) * nb + bx) < thr) return false;
-            exit_t = box_exit(g, n, bx * 8, bx * 8 + 8, by * 8, by * 8 + 8, bz * 8, bz * 8 + 8, st.far_d);
-        }
-    }
+    const int nb = S->nb, bx = vx >> 3, by = vy >> 3, bz = vz >> 3;   // (n / 8)^3 bricks: 32-bit indices
+    int early = 0;
+    if constexpr (kEager) early = ld_keep(S->sdil + ((vz >> 5) * S->ns + (vy >> 5)) * S->ns + (vx >> 5));
+    if (__ldg(S->bdil + (bz * nb + by) * nb + bx) < thr) return false;
+    const int n = S->n, ns = S->ns, sx = vx >> 5, sy = vy >> 5, sz = vz >> 5;
+    const float exit_t = (kEager ? early : __ldg(S->sdil + (sz * ns + sy) * ns + sx)) >= thr
+                             ? superbrick_run_exit(S, g, thr, sx, sy, sz, st.far_d)
+                             : box_exit(g, n, bx * 8, bx * 8 + 8, by * 8, by * 8 + 8, bz * 8, bz * 8 + 8, st.far_d);
     // skip this sample and every later one whose base voxel stays in the box
     skip_to(st, fminf(exit_t, st.far_d), inc);
     return true;
@@ -476,14 +475,31 @@ __device__ int march_serial(const SessionDev* S, const RayGeo& g, const TF* f, R
         const float inc = st.small ? small : large;
         float x, y, z;
         texel(g, st.t, x, y, z);
-        const TexelBase tb = texel_base(n, x, y, z);
+        const InnerBase b = inner_base(n, x, y, z);
         const int g0 = st.guard;
-        if (bdil && skip_cell<kEager>(S, g, st, tb.x0, tb.y0, tb.z0, inc)) {
+        bool skipped;
+        if constexpr (kEager) {
+            int vx = b.x0, vy = b.y0, vz = b.z0;
+            if (!b.in) clamp_voxel(n, vx, vy, vz);
+            skipped = bdil && skip_cell<true>(S, g, st, vx, vy, vz, inc);
+        } else {   // in 64 registers two copies of the skip spill less than clamped copies of the voxel
+            skipped = false;
+            if (bdil) {
+                if (b.in) {
+                    skipped = skip_cell<false>(S, g, st, b.x0, b.y0, b.z0, inc);
+                } else {
+                    const TexelBase tb = texel_base(n, x, y, z);
+                    skipped = skip_cell<false>(S, g, st, tb.x0, tb.y0, tb.z0, inc);
+                }
+            }
+        }
+        if (skipped) {
             cnt.add(kCntSkips, 1u);
             cnt.add(kCntSkipped, unsigned(st.guard - g0));
             continue;
         }
-        const float tsdf = trilinear_at(f, n, tb);
+        const float tsdf = b.in ? trilinear_inner(f, unsigned(n), voxel_index(unsigned(n), b.x0, b.y0, b.z0), b.ax, b.ay, b.az)
+                                : trilinear(f, n, x, y, z);
         cnt.add(st.small ? kCntEvalSmall : kCntEvalLarge, 1u);
         ++st.guard;
         if (tsdf < 0.0f) {
@@ -493,11 +509,7 @@ __device__ int march_serial(const SessionDev* S, const RayGeo& g, const TF* f, R
                     begin_small(st, __fsub_rn(st.t, mu), small);
                     continue;
                 }
-                if (!st.prev_known) {
-                    float px, py, pz;
-                    texel(g, st.prev_t, px, py, pz);
-                    st.prev = trilinear(f, n, px, py, pz);
-                }
+                if (!st.prev_known) st.prev = sample_at(S, g, f, st.prev_t);
                 precise = st.t - small * st.prev / (tsdf - st.prev);   // the reference's formula
             }
             return 1;
@@ -533,9 +545,11 @@ __device__ void march_coop(const SessionDev* S, const RayGeo& g, const TF* f, Ra
         if (S->bdil) {
             float x, y, z;
             texel(g, st.t, x, y, z);
-            const TexelBase tb = texel_base(S->n, x, y, z);
+            const InnerBase b = inner_base(S->n, x, y, z);
+            int vx = b.x0, vy = b.y0, vz = b.z0;
+            if (!b.in) clamp_voxel(S->n, vx, vy, vz);
             const int g0 = st.guard;
-            if (skip_cell<true>(S, g, st, tb.x0, tb.y0, tb.z0, inc)) {   // every lane takes the same steps
+            if (skip_cell<true>(S, g, st, vx, vy, vz, inc)) {   // every lane takes the same steps
                 if (lane == 0) {
                     cnt.add(kCntSkips, 1u);
                     cnt.add(kCntSkipped, unsigned(st.guard - g0));
@@ -659,6 +673,40 @@ __device__ __forceinline__ float grad_sample(const TF* f, int n, const HitGeo& h
                      a == 2 ? __fadd_rn(h.z, d) : h.z);
 }
 
+// The six samples of a hit whose taps all lie inside the volume (almost every one) share the base
+// voxel and the weights of the two axes they do not move along, and clamp nothing; the others take
+// grad_sample's general form.
+template <class TF>
+__device__ __forceinline__ void grad_samples(const TF* f, int n, const HitGeo& h, float (&v)[6]) {
+    const InnerBase b = inner_base(n, h.x, h.y, h.z);
+    float ax[6];
+    int d[6];   // base voxel of sample q along its axis
+    unsigned int far = 0;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        const int a = q < 3 ? q : q - 3;
+        d[q] = floor_split(__fadd_rn(a == 0 ? h.x : a == 1 ? h.y : h.z, q < 3 ? h.rt : -h.rt), ax[q]);
+        far = max(far, unsigned(d[q]));
+    }
+    if (b.in && far < unsigned(n - 1)) {
+        const unsigned int un = unsigned(n), idx = voxel_index(un, b.x0, b.y0, b.z0);
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            const int a = q < 3 ? q : q - 3;
+            const unsigned int at = idx + unsigned(d[q] - (a == 0 ? b.x0 : a == 1 ? b.y0 : b.z0)) * (a == 0 ? 1u : a == 1 ? un : un * un);
+            v[q] = trilinear_inner(f, un, at, a == 0 ? ax[q] : b.ax, a == 1 ? ax[q] : b.ay, a == 2 ? ax[q] : b.az);
+        }
+        return;
+    }
+#pragma unroll 1
+    for (int q = 0; q < 6; ++q) {
+        const float w = grad_sample(f, n, h, q);
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+            if (k == q) v[k] = w;
+    }
+}
+
 // the normal from the six samples and the map writes (project/src/raycast.cu:120-144)
 __device__ __forceinline__ void write_hit(const SessionDev* S, int level, int i, int j, bool hit, const HitGeo& h,
                                           const float (&v)[6]) {
@@ -692,8 +740,7 @@ __device__ void finish_ray(const SessionDev* S, const RayGeo& g, const TF* f, in
     float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (precise != 0.0f) {
         cnt.add(kCntGrad, 6u);
-#pragma unroll
-        for (int q = 0; q < 6; ++q) v[q] = grad_sample(f, S->n, h, q);
+        grad_samples(f, S->n, h, v);
     }
     write_hit(S, level, i, j, precise != 0.0f, h, v);
 }
@@ -838,7 +885,7 @@ __global__ void __launch_bounds__(256) ray_range_kernel(EngineView v) {
 // Each warp pulls 8 x 4-ray tiles on its own (no block-wide barrier).  Steps of many ray tiles
 // run four blocks per SM (64 registers: more warps to hide the gathers behind); a single
 // session's step runs three (80 registers: fewer instructions per sample, a shorter tail).
-template <int kBlocksPerSm, bool kCount>
+template <int kBlocksPerSm, bool kCount, int kFmt>
 __global__ void __launch_bounds__(256, kBlocksPerSm) raycast_kernel(EngineView v) {
     MarchCount<kCount> cnt;
     const int lane = threadIdx.x & 31;
@@ -862,7 +909,7 @@ __global__ void __launch_bounds__(256, kBlocksPerSm) raycast_kernel(EngineView v
         float m[9];
         F3 o;
         ray_matrix(S, Lv, m, o);
-        if (S->fmt == KF_TSDF_F16U16)
+        if (kFmt == KF_TSDF_F16U16 || (kFmt == kAnyFormat && S->fmt == KF_TSDF_F16U16))
             serial_ray<__half, MarchCount<kCount>, kBlocksPerSm == 3>(rq, S, T.s, m, o, T.level, i, j, budget, cnt);
         else
             serial_ray<float, MarchCount<kCount>, kBlocksPerSm == 3>(rq, S, T.s, m, o, T.level, i, j, budget, cnt);
@@ -908,14 +955,23 @@ cudaError_t launch_ray_range(const EngineView& v, int grid, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_raycast(const EngineView& v, int grid, cudaStream_t st, bool many) {
+template <int kFmt>
+static void launch_tiles(const EngineView& v, int grid, cudaStream_t st, bool many) {
+    if (many) raycast_kernel<4, false, kFmt><<<grid, 256, 0, st>>>(v);
+    else raycast_kernel<3, false, kFmt><<<grid, 256, 0, st>>>(v);
+}
+
+cudaError_t launch_raycast(const EngineView& v, int grid, int fmt, cudaStream_t st, bool many) {
     const bool count = v.ray_counts != nullptr;
     if (count) {
-        if (many) raycast_kernel<4, true><<<grid, 256, 0, st>>>(v);
-        else raycast_kernel<3, true><<<grid, 256, 0, st>>>(v);
+        if (many) raycast_kernel<4, true, kAnyFormat><<<grid, 256, 0, st>>>(v);
+        else raycast_kernel<3, true, kAnyFormat><<<grid, 256, 0, st>>>(v);
+    } else if (fmt == KF_TSDF_F32F32) {
+        launch_tiles<KF_TSDF_F32F32>(v, grid, st, many);
+    } else if (fmt == KF_TSDF_F16U16) {
+        launch_tiles<KF_TSDF_F16U16>(v, grid, st, many);
     } else {
-        if (many) raycast_kernel<4, false><<<grid, 256, 0, st>>>(v);
-        else raycast_kernel<3, false><<<grid, 256, 0, st>>>(v);
+        launch_tiles<kAnyFormat>(v, grid, st, many);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;

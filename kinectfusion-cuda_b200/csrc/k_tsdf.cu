@@ -276,10 +276,6 @@ __device__ __forceinline__ void fuse_half(const FuseCtx& c, int x0, int j0, int 
     }
 }
 
-// The fusion kernels are built for volumes of one format, with the registers that format needs, and
-// for batches of both (kAnyFormat).
-constexpr int kAnyFormat = -1;
-
 // part `part` of `split` (1, 2 or 4) of packed half unit b
 template <int kFmt>
 __device__ __forceinline__ void fuse_part(const FuseCtx& c, unsigned int b, unsigned int part, unsigned int split, int lane) {

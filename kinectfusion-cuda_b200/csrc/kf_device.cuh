@@ -249,6 +249,20 @@ __device__ __forceinline__ TexelBase texel_base(int n, float x, float y, float z
     return b;
 }
 
+// the seven lerps of a trilinear sample, each a (1 - w) + b w as one rounded product and one fused
+// multiply-add, spelled out so every kernel that samples the volume rounds identically
+__device__ __forceinline__ float lerp8(float v000, float v100, float v010, float v110, float v001, float v101, float v011,
+                                       float v111, float ax, float ay, float az) {
+    const float bx = __fsub_rn(1.f, ax), by = __fsub_rn(1.f, ay), bz = __fsub_rn(1.f, az);
+    const float c00 = __fmaf_rn(v100, ax, __fmul_rn(v000, bx));
+    const float c10 = __fmaf_rn(v110, ax, __fmul_rn(v010, bx));
+    const float c01 = __fmaf_rn(v101, ax, __fmul_rn(v001, bx));
+    const float c11 = __fmaf_rn(v111, ax, __fmul_rn(v011, bx));
+    const float c0 = __fmaf_rn(c10, ay, __fmul_rn(c00, by));
+    const float c1 = __fmaf_rn(c11, ay, __fmul_rn(c01, by));
+    return __fmaf_rn(c1, az, __fmul_rn(c0, bz));
+}
+
 // trilinear sample of the distance array from its base voxel: what tex3D<float2>(...).x
 // returns with normalized coordinates, linear filtering and clamp addressing
 // (project/src/voxel_grid.cpp:24-33), computed with exact float weights.  n^3 < 2^32, so the
@@ -263,26 +277,51 @@ __device__ __forceinline__ float trilinear_at(const TF* f, int n, const TexelBas
     const TF* p10 = p00 + dy;
     const TF* p01 = p00 + dz;
     const TF* p11 = p01 + dy;
-    const float v000 = load_f(p00, 0), v100 = load_f(p00, dx);
-    const float v010 = load_f(p10, 0), v110 = load_f(p10, dx);
-    const float v001 = load_f(p01, 0), v101 = load_f(p01, dx);
-    const float v011 = load_f(p11, 0), v111 = load_f(p11, dx);
-    // each lerp a (1 - w) + b w as one rounded product and one fused multiply-add, spelled
-    // out so every kernel that samples the volume rounds identically
-    const float bx = __fsub_rn(1.f, b.ax), by = __fsub_rn(1.f, b.ay), bz = __fsub_rn(1.f, b.az);
-    const float c00 = __fmaf_rn(v100, b.ax, __fmul_rn(v000, bx));
-    const float c10 = __fmaf_rn(v110, b.ax, __fmul_rn(v010, bx));
-    const float c01 = __fmaf_rn(v101, b.ax, __fmul_rn(v001, bx));
-    const float c11 = __fmaf_rn(v111, b.ax, __fmul_rn(v011, bx));
-    const float c0 = __fmaf_rn(c10, b.ay, __fmul_rn(c00, by));
-    const float c1 = __fmaf_rn(c11, b.ay, __fmul_rn(c01, by));
-    return __fmaf_rn(c1, b.az, __fmul_rn(c0, bz));
+    return lerp8(load_f(p00, 0), load_f(p00, dx), load_f(p10, 0), load_f(p10, dx), load_f(p01, 0), load_f(p01, dx),
+                 load_f(p11, 0), load_f(p11, dx), b.ax, b.ay, b.az);
 }
 
 // trilinear sample at texel coordinates (x, y, z)
 template <class TF>
 __device__ __forceinline__ float trilinear(const TF* f, int n, float x, float y, float z) {
     return trilinear_at(f, n, texel_base(n, x, y, z));
+}
+
+// floor(x) as an integer, and its remainder, for |x| < 2^22: the sum with 1.5 * 2^23 rounded down holds
+// the floor in its low bits.  Two additions in place of the two conversions of floorf and the cast,
+// with the same results; any other x gives an integer outside [0, 2^22).
+__device__ __forceinline__ int floor_split(float x, float& frac) {
+    const float t = __fadd_rd(x, 12582912.0f);
+    frac = __fsub_rn(x, __fsub_rn(t, 12582912.0f));
+    return __float_as_int(t) - 0x4B400000;
+}
+
+// A sample whose eight taps all lie inside the volume, so that no tap clamps: almost every one.  `in`
+// says so; the others go through TexelBase.
+struct InnerBase {
+    float ax, ay, az;
+    int x0, y0, z0;
+    bool in;
+};
+
+__device__ __forceinline__ InnerBase inner_base(int n, float x, float y, float z) {
+    InnerBase b;
+    b.x0 = floor_split(x, b.ax);
+    b.y0 = floor_split(y, b.ay);
+    b.z0 = floor_split(z, b.az);
+    b.in = max(max(unsigned(b.x0), unsigned(b.y0)), unsigned(b.z0)) < unsigned(n - 1);
+    return b;
+}
+
+// the sample of base voxel `idx` (linear) with the given weights; taps inside the volume
+template <class TF>
+__device__ __forceinline__ float trilinear_inner(const TF* f, unsigned int n, unsigned int idx, float ax, float ay, float az) {
+    const TF* p00 = f + idx;
+    const TF* p10 = p00 + n;
+    const TF* p01 = p00 + n * n;
+    const TF* p11 = p01 + n;
+    return lerp8(load_f(p00, 0), load_f(p00, 1), load_f(p10, 0), load_f(p10, 1), load_f(p01, 0), load_f(p01, 1),
+                 load_f(p11, 0), load_f(p11, 1), ax, ay, az);
 }
 
 // globaltimer (ns) for bounded waits

@@ -25,6 +25,9 @@ struct Tables {
     long long vis_fuse_total;  // the same over the slots' visualization volumes
 };
 
+// The raycast and fusion kernels are built for volumes of one format, with the registers that format
+// needs, and for slots of both (kAnyFormat); the launches take the format every slot has.
+constexpr int kAnyFormat = -1;
 constexpr int kCounters = 12;   // words of EngineView::counters
 
 struct LongRay;   // march state of a ray handed from a lane to a warp (k_raycast.cu)
@@ -107,12 +110,11 @@ cudaError_t launch_preprocess(const EngineView& v, int grid, cudaStream_t st);
 // The depth ranges of a step's raycast (a grid of one thread per fusion unit, or grid-stride); also
 // clears the wait record and the counters.
 cudaError_t launch_ray_range(const EngineView& v, int grid, cudaStream_t st);
-cudaError_t launch_raycast(const EngineView& v, int grid, cudaStream_t st, bool many);
+cudaError_t launch_raycast(const EngineView& v, int grid, int fmt, cudaStream_t st, bool many);
 int serial_budget_many();   // the lane budget of the raycast's many-tile form
 int ray_count_slots();      // entries of the raycast's debug work counts
 // single: an engine of one slot (the kernel keeps that session's state per block)
 cudaError_t launch_icp(const EngineView& v, int grid, cudaStream_t st, bool single);
-// fmt: the volume format every slot has, or -1 for slots of both
 cudaError_t launch_fuse(const EngineView& v, int grid, int fmt, cudaStream_t st);
 // the constant part of a session's fusion context (its tracking or its visualization volume)
 FuseCtx fuse_context(const SessionDev& d, bool vis);
