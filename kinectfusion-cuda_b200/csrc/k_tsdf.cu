@@ -121,7 +121,11 @@ __device__ __forceinline__ bool block_culled(const FuseCtx& c, int x0, int nx, i
     const int tx1 = min(max(int(pxmax + 0.01f), 0), c.w - 1) >> 4;
     const int ty0 = min(max(int(pymin - 0.01f), 0), c.h - 1) >> 4;
     const int ty1 = min(max(int(pymax + 0.01f), 0), c.h - 1) >> 4;
-    if ((tx1 - tx0 + 1) * (ty1 - ty0 + 1) > 512) return false;
+    // A box over many tiles is near the camera or coarse, and seldom behind every depth under it; one
+    // thread reading them all held the launch (frame and visualization volume of 256^3 over 8 m and
+    // 512^3 over 5 m, cull + cull: 28 + 13 us with up to 512 tiles, 12 + 11 with 32, 11 + 10 with 8, where
+    // fusion takes 10 us more; 512^3 over 3 m the same with 32 and 512).
+    if ((tx1 - tx0 + 1) * (ty1 - ty0 + 1) > 32) return false;
     float dm = 0.0f;
     for (int ty = ty0; ty <= ty1; ++ty)
         for (int tx = tx0; tx <= tx1; ++tx) dm = fmaxf(dm, __ldg(c.dmax + size_t(ty) * c.t16w + tx));
