@@ -195,3 +195,61 @@ def test_session_fusion_equals_the_stage(kf, cuda, sizes):
         assert n == 8 or (w > 0).any()
         alone.close()
     b.close()
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (31, 7), (33, 9), (161, 119), (64, 8)])
+def test_icp_rows_shapes(kf, orc, cuda, w, h):
+    """Residual rows in sizes that the kernel's 32 x 8-pixel blocks do not divide: the float oracle's
+    rows to a relative 1e-5 of the largest entry (both in float, a few fused roundings apart), the
+    same zero rows but for pixels within rounding of a rejection (at most 1 %), nothing written past
+    the end."""
+    from kfb200 import synth
+    cfg = kf.config_small(width=max(w, 2), height=max(h, 2), fx=262.5 * w / 320, fy=262.5 * w / 320, cx=w / 2 - 0.5,
+                          cy=h / 2 - 0.5, levels=1)
+    poses = synth.trajectory(synth.LOOP, 6, 4, cfg.volume_width)
+    k = kf.level_intrinsics(cfg, 0)
+    ik = np.linalg.inv(k.astype(np.float64)).astype(np.float32)
+    vm = []
+    for i in (4, 5):
+        img = synth.render(synth.scene(cfg.volume_width), poses[i], w, h, float(cfg.fx), float(cfg.fy), float(cfg.cx),
+                           float(cfg.cy), 4, i, noise=False)
+        vm.append(orc.vertex_map(orc.convert(img, 1e-3), ik))
+    tv, tn = vm[0].copy(), orc.normal_map(vm[0])
+    R, t = poses[4][:3, :3], poses[4][:3, 3]
+    tv[..., :3] = np.where(tv[..., 3:] == -1, tv[..., :3] @ R.T + t, 0)
+    tn[..., :3] = np.where(tn[..., 3:] == -1, tn[..., :3] @ R.T, 0)
+    rows = w * h
+    A = cuda.full((rows * 6 + 8,), 7.0, device="cuda")
+    b = cuda.full((rows + 8,), 7.0, device="cuda")
+    kf.kernel.constructIcpResiduals(dev(cuda, vm[1]), dev(cuda, tv), dev(cuda, tn), R, t, R, t, k, 0.1, 0.35, A, b)
+    oa, ob = orc.icp_residuals(vm[1], tv, tn, R, t, R, t, k, 0.1, 0.35)[:2]
+    ga, gb = A[:rows * 6].cpu().numpy().reshape(-1, 6), b[:rows].cpu().numpy()
+    assert float((A[rows * 6:] - 7).abs().max()) == 0 and float((b[rows:] - 7).abs().max()) == 0
+    oa, ob = np.asarray(oa).reshape(-1, 6), np.asarray(ob).reshape(-1)
+    flips = (np.abs(ga).sum(1) == 0) != (np.abs(oa).sum(1) == 0)
+    assert flips.sum() <= 0.01 * rows
+    scale = max(1.0, float(np.abs(oa).max(initial=0)))
+    assert np.abs(ga - oa)[~flips].max(initial=0) <= 1e-5 * scale
+    assert np.abs(gb - ob)[~flips].max(initial=0) <= 1e-5 * scale
+
+
+@pytest.mark.parametrize("n", [1, 6, 255, 256, 257, 2047, 2049, 8193, 148 * 4 * 2048 + 5])
+def test_least_squares_alignments_agree(kf, cuda, n):
+    """A that starts on 8 bytes (read in pairs) and the same rows 4 bytes further: the same sums in
+    the same order, so the same x bit for bit (or the same failure, for too few rows)."""
+    import ctypes
+    g = cuda.Generator(device="cuda").manual_seed(n)
+    rows = cuda.randn((n, 6), device="cuda", generator=g)
+    b = cuda.randn((n,), device="cuda", generator=g)
+    room = cuda.zeros(6 * n + 1, device="cuda")
+    room[1:] = rows.reshape(-1)
+    got = []
+    for at in (rows.data_ptr(), room.data_ptr() + 4):
+        x = (ctypes.c_float * 6)()
+        st = kf.lib.kf_solve_linear_least_squares(ctypes.c_void_p(at), ctypes.c_void_p(b.data_ptr()), n, x, None)
+        got.append((st, np.array(x[:], np.float32).view(np.int32).tolist()))
+    assert got[0] == got[1]
+    if n >= 255:
+        a64, b64 = rows.double().cpu().numpy(), b.double().cpu().numpy()
+        want = np.linalg.solve(a64.T @ a64, a64.T @ b64)
+        np.testing.assert_allclose(np.array(got[0][1], np.int32).view(np.float32), want, rtol=1e-4, atol=1e-6)
