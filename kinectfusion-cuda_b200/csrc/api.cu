@@ -190,7 +190,6 @@ struct Slot {
     int frames = 0;
     kf_frame_stats stats{};
     float pose[16]{};
-    bool external = false;   // maps supplied by the caller (kf_compute_pose)
     float4* render_v = nullptr;          // kf_render's own level-0 maps and image (lazily)
     float4* render_n = nullptr;
     unsigned int* render_rgba = nullptr;
@@ -237,7 +236,6 @@ struct Slot {
         render_rgba = nullptr;
         bytes = 0;
         used = false;
-        external = false;
         frames = 0;
     }
 };
@@ -269,6 +267,18 @@ void fill_levels(SessionDev& d, const kf_config& c) {
     d.angle_cos = float(std::cos(double(c.angle_thresh)));
     d.stop_a = c.stop_angle;
     d.stop_d = c.stop_dist;
+}
+
+// The ICP tiles of one session-level: up to a few per ICP block (the grid's blocks take them round
+// robin, which evens out tiles of mostly invalid pixels), each at least one pipelined step of the block
+// (kIcpMinTile pixels): small levels get few tiles, so a pass over many sessions stores few partials.
+void icp_tiles(const LevelDev& Lv, int s, std::vector<IcpTile>& out) {
+    const int np = Lv.icw * Lv.ich;
+    const int per_block = std::max(1, std::min(kIcpTilesPerBlock, np / (kIcpGroups * kIcpMinTile)));
+    const int ntiles = kIcpGroups * per_block;
+    int tile = (np + ntiles - 1) / ntiles;
+    tile = std::max(kIcpMinTile, (tile + 31) / 32 * 32);
+    for (int p0 = 0; p0 < np; p0 += tile) out.push_back(IcpTile{s, p0, std::min(tile, np - p0)});
 }
 
 // allocate and initialise a session's buffers; all device work on st, synchronised before
@@ -656,7 +666,7 @@ struct Engine {
     void destroy() {
         if (gexec) cudaGraphExecDestroy(gexec);
         gexec = nullptr;
-        for (Slot& s : slots) if (!s.external) s.release();
+        for (Slot& s : slots) s.release();
         for (cudaEvent_t& e : ev)
             if (e) cudaEventDestroy(e);
         cudaFree(d_sess); cudaFree(d_fctx); cudaFree(d_step); cudaFree(d_out); cudaFree(d_tb); cudaFree(d_pre); cudaFree(d_ray);
@@ -770,35 +780,21 @@ struct Engine {
             max_levels = std::max(max_levels, c.levels);
             range |= sl.d.range != nullptr;
             formats |= 1 << sl.d.fmt;
-            if (!sl.external) {
-                for (int y = 0; y < c.height; y += kPreTileSize)
-                    for (int x = 0; x < c.width; x += kPreTileSize) pre.push_back(PreTile{s, x, y});
-                for (int l = 0; l < c.levels; ++l) {
-                    const LevelDev& Lv = sl.d.lv[l];
-                    const int tw = shape.ray_tw, th = 32 / shape.ray_tw;
-                    for (int y = 0; y < Lv.ch; y += th)
-                        for (int x = 0; x < Lv.cw; x += tw) ray.push_back(RayTile{s, l, x, y});
-                }
-                fprefix[s + 1] += fuse_units(c.volume_n);
-                if (sl.d.vis.n) vfprefix[s + 1] += fuse_units(sl.d.vis.n);
-            }
+            for (int y = 0; y < c.height; y += kPreTileSize)
+                for (int x = 0; x < c.width; x += kPreTileSize) pre.push_back(PreTile{s, x, y});
             for (int l = 0; l < c.levels; ++l) {
                 const LevelDev& Lv = sl.d.lv[l];
-                const int np = Lv.icw * Lv.ich;
-                // up to a few tiles per ICP block per session-level (the grid's blocks take them
-                // round robin, which evens out tiles of mostly invalid pixels), each at least
-                // one pipelined step of the block (kIcpMinTile pixels): small levels get few
-                // tiles, so a pass over many sessions stores few partials
-                const int per_block = std::max(1, std::min(kIcpTilesPerBlock, np / (kIcpGroups * kIcpMinTile)));
-                const int ntiles = kIcpGroups * per_block;
-                int tile = (np + ntiles - 1) / ntiles;
-                tile = std::max(kIcpMinTile, (tile + 31) / 32 * 32);
+                const int tw = shape.ray_tw, th = 32 / shape.ray_tw;
+                for (int y = 0; y < Lv.ch; y += th)
+                    for (int x = 0; x < Lv.cw; x += tw) ray.push_back(RayTile{s, l, x, y});
                 IcpRange rg;
                 rg.begin = int(it[l].size());
-                for (int p0 = 0; p0 < np; p0 += tile) it[l].push_back(IcpTile{s, p0, std::min(tile, np - p0)});
+                icp_tiles(Lv, s, it[l]);
                 rg.end = int(it[l].size());
                 ranges[size_t(l) * cap + s] = rg;
             }
+            fprefix[s + 1] += fuse_units(c.volume_n);
+            if (sl.d.vis.n) vfprefix[s + 1] += fuse_units(sl.d.vis.n);
         }
         // concatenate ICP levels; ranges become absolute
         std::vector<IcpTile> all;
@@ -1663,7 +1659,6 @@ kf_status kf_render(kf_session* s, int mode, const float pose_in[16], uint8_t* r
     NvtxRange nvtx_("kf_render");
     if (!s || !rgba || (mode != KF_RENDER_NORMALS && mode != KF_RENDER_SHADING)) return KF_ERR_ARG;
     Slot& sl = s->sl();
-    if (sl.external) return KF_ERR_STATE;
     const kf_config& c = sl.cfg;
     const int w = c.width, h = c.height;
     cudaStream_t st = as_stream(stream);
@@ -1913,50 +1908,85 @@ kf_status kf_compute_pose(const float* const* vertex, const float* const* target
     if (total > kIcpMaxPasses) return KF_ERR_ARG;
     for (int l = 0; l < levels; ++l)
         if (!vertex[l] || !target_vertex[l] || !target_normal[l]) return KF_ERR_ARG;
-    Engine eng;
-    kf_status st = eng.init(1);
-    if (st != KF_OK) { eng.destroy(); return st; }
-    Slot& sl = eng.slots[0];
-    sl.cfg = c;
-    sl.used = true;
-    sl.external = true;
-    std::memset(&sl.d, 0, sizeof(sl.d));
-    fill_levels(sl.d, c);
-    for (int l = 0; l < levels; ++l) {
-        sl.d.vmap[l] = reinterpret_cast<float4*>(const_cast<float*>(vertex[l]));
-        sl.d.pv[l] = reinterpret_cast<float4*>(const_cast<float*>(target_vertex[l]));
-        sl.d.pn[l] = reinterpret_cast<float4*>(const_cast<float*>(target_normal[l]));
-    }
-    PoseDev* d_pose = nullptr;
     cudaStream_t s = as_stream(stream);
-    auto fail = [&](cudaError_t e) {
-        g_last_cuda = e;
-        if (d_pose) cudaFree(d_pose);
-        eng.destroy();
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    KF_CK(cudaStreamIsCapturing(s, &cs));
+    if (cs != cudaStreamCaptureStatusNone) {   // the pose comes back to the host: not capturable
+        g_last_cuda = cudaErrorStreamCaptureUnsupported;
         return KF_ERR_CUDA;
+    }
+    // maps written on the default stream may be passed with any stream
+    if (s) KF_CK(cudaStreamSynchronize(nullptr));
+
+    // One block of scratch, whose head [session | step | tables | tile ranges | pose | sync, result |
+    // tiles] is filled here and copied at once; the kernel writes the rest before it reads it: 85 us at
+    // 640x480 and three levels, most of it the ICP launch.  An engine made and destroyed per call, with
+    // some twenty allocations and their frees, three streams and ten copies, took 0.6 to 8 ms.
+    std::vector<IcpTile> tiles;
+    IcpRange ranges[KF_MAX_LEVELS] = {};
+    SessionDev d;
+    std::memset(&d, 0, sizeof(d));
+    fill_levels(d, c);
+    for (int l = 0; l < levels; ++l) {
+        d.vmap[l] = reinterpret_cast<float4*>(const_cast<float*>(vertex[l]));
+        d.pv[l] = reinterpret_cast<float4*>(const_cast<float*>(target_vertex[l]));
+        d.pn[l] = reinterpret_cast<float4*>(const_cast<float*>(target_normal[l]));
+        ranges[l].begin = int(tiles.size());
+        icp_tiles(d.lv[l], 0, tiles);
+        ranges[l].end = int(tiles.size());
+    }
+    size_t bytes = 0;
+    const auto part = [&bytes](size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255) & ~size_t(255);
+        return at;
     };
-    cudaError_t e = cudaMalloc(&d_pose, sizeof(PoseDev));
-    if (e != cudaSuccess) return fail(e);
-    PoseDev P = make_pose_dev(pose);
-    e = cudaMemcpy(d_pose, &P, sizeof(P), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return fail(e);
-    sl.d.pose = d_pose;
-    st = eng.build_tables();
-    if (st != KF_OK) { cudaFree(d_pose); eng.destroy(); return st; }
-    StepDev step{1, 0};
-    e = cudaMemcpy(eng.d_step, &step, sizeof(step), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemsetAsync(eng.d_sync, 0, sizeof(GridSync), s);
-    if (e == cudaSuccess) e = launch_icp(eng.view(), eng.shape.grid_icp, s, eng.cap == 1);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(eng.h_out, eng.d_out, eng.out_bytes(), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return fail(e);
-    std::memcpy(pose_out, eng.h_out[0].pose, sizeof(float) * 16);
+    const size_t o_sess = part(sizeof(SessionDev)), o_step = part(sizeof(StepDev)), o_tb = part(sizeof(Tables)),
+                 o_ranges = part(sizeof(ranges)), o_pose = part(sizeof(PoseDev)),
+                 o_out = part(sizeof(OutDev) + sizeof(GridSync)), o_tiles = part(sizeof(IcpTile) * tiles.size());
+    const size_t head = bytes;
+    const size_t o_fctx = part(2 * sizeof(FuseCtx)), o_parts = part(2 * tiles.size() * kIcpPartialStride * sizeof(float));
+    Scratch scratch;
+    KF_CK(scratch.take(bytes, s));
+    char* const base = static_cast<char*>(scratch.p);
+    std::vector<char> host(head, 0);
+    const auto put = [&host](size_t at, const void* src, size_t n) { std::memcpy(host.data() + at, src, n); };
+    d.pose = reinterpret_cast<PoseDev*>(base + o_pose);
+    Tables tb{};
+    tb.S = 1;
+    tb.max_levels = levels;
+    const StepDev step{1, 0};
+    const PoseDev P = make_pose_dev(pose);
+    put(o_sess, &d, sizeof(d));
+    put(o_step, &step, sizeof(step));
+    put(o_tb, &tb, sizeof(tb));
+    put(o_ranges, ranges, sizeof(ranges));
+    put(o_pose, &P, sizeof(P));
+    put(o_tiles, tiles.data(), sizeof(IcpTile) * tiles.size());
+    EngineView v{};
+    v.sess = reinterpret_cast<SessionDev*>(base + o_sess);
+    v.step = reinterpret_cast<StepDev*>(base + o_step);
+    v.tb = reinterpret_cast<Tables*>(base + o_tb);
+    v.iranges = reinterpret_cast<IcpRange*>(base + o_ranges);
+    v.out = reinterpret_cast<OutDev*>(base + o_out);
+    v.sync = reinterpret_cast<GridSync*>(v.out + 1);
+    v.itiles = reinterpret_cast<IcpTile*>(base + o_tiles);
+    v.fctx = reinterpret_cast<FuseCtx*>(base + o_fctx);
+    v.vis_fctx = v.fctx + 1;
+    v.partials = reinterpret_cast<float*>(base + o_parts);
+    v.partials2 = v.partials + tiles.size() * kIcpPartialStride;
+    int dev = 0, sms = 0;
+    KF_CK(cudaGetDevice(&dev));
+    KF_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    struct { OutDev out; GridSync sync; } res;
+    KF_CK(cudaMemcpyAsync(base, host.data(), head, cudaMemcpyHostToDevice, s));
+    KF_CK(launch_icp(v, sms, s, true));
+    KF_CK(cudaMemcpyAsync(&res, v.out, sizeof(res), cudaMemcpyDeviceToHost, s));
+    KF_CK(cudaStreamSynchronize(s));
+    std::memcpy(pose_out, res.out.pose, sizeof(float) * 16);
     if (iters_out)
-        for (int l = 0; l < KF_MAX_LEVELS; ++l) iters_out[l] = eng.h_out[0].iters[l];
-    kf_status r = eng.h_sync->abort ? KF_ERR_TIMEOUT : kf_status(eng.h_out[0].status);
-    cudaFree(d_pose);
-    eng.destroy();
-    return r;
+        for (int l = 0; l < KF_MAX_LEVELS; ++l) iters_out[l] = res.out.iters[l];
+    return res.sync.abort ? KF_ERR_TIMEOUT : kf_status(res.out.status);
 }
 
 kf_status kf_pose_error(const float p1[16], const float p2[16], float out[2]) {
@@ -2657,7 +2687,6 @@ kf_status kf_session_stage_times(kf_session* s, float ms[4]) {
 
 // debug modes of one slot's session (traces) and of its engine (plain launches)
 static kf_status slot_set_debug(Engine& e, Slot& sl, int flags) {
-    if (sl.external) return KF_ERR_STATE;
     const bool want = (flags & KF_DEBUG_RAY_TRACE) != 0;
     for (int l = 0; l < sl.cfg.levels; ++l) {
         if (want && !sl.d.trace[l]) {

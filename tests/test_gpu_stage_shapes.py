@@ -253,3 +253,40 @@ def test_least_squares_alignments_agree(kf, cuda, n):
         a64, b64 = rows.double().cpu().numpy(), b.double().cpu().numpy()
         want = np.linalg.solve(a64.T @ a64, a64.T @ b64)
         np.testing.assert_allclose(np.array(got[0][1], np.int32).view(np.float32), want, rtol=1e-4, atol=1e-6)
+
+
+@pytest.mark.parametrize("w,h,levels,side", [(32, 24, 1, False), (36, 28, 3, False), (164, 124, 2, True),
+                                             (320, 240, 3, False), (640, 480, 3, True)])
+def test_compute_pose_equals_the_session(kf, cuda, w, h, levels, side):
+    """ICP.computePose on a session's own maps gives the session's pose and iterations bit for bit
+    (its second frame: the start pose is the configuration's), on the default stream and on another,
+    with calls that follow one another and calls of two threads at once."""
+    import threading
+    from kfb200 import synth
+    cfg = kf.config_small(width=w, height=h, fx=262.5 * w / 320, fy=262.5 * w / 320, cx=w / 2 - 0.5, cy=h / 2 - 0.5,
+                          levels=levels, iters=(6, 4, 3)[:levels], volume_n=64, mu=0.06)
+    imgs, _ = synth.sequence(cfg, 2, seed=3, kind=synth.LOOP)
+    s = kf.KinectFusion(cfg)
+    s.process_frame(imgs[0])
+    status, pose = s.process_frame(imgs[1])
+    iters = s.frame_stats()["icp_iters"]
+    maps = [[dev(cuda, m) for m in (s.vertex_map(lv), *s.raycast_maps(lv))] for lv in range(levels)]
+    start = np.array(list(cfg.initial_pose), np.float32).reshape(4, 4).T
+    out = []
+
+    def call():
+        stream = cuda.cuda.Stream() if side else None
+        for _ in range(3):
+            out.append(kf.ICP(cfg).computePose(*[[m[k] for m in maps] for k in range(3)], start, stream=stream))
+    call()
+    threads = [threading.Thread(target=call) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(out) == 9
+    for st, p, it in out:
+        assert st == status and it == iters
+        if st == 0:
+            np.testing.assert_array_equal(p.view(np.int32), np.asarray(pose, np.float32).view(np.int32))
+    s.close()
