@@ -883,6 +883,17 @@ struct Engine {
             if (stages[0]) KF_CK(launch_preprocess(v, shape.grid_pre, st));
             if (profile) KF_CK(cudaEventRecordWithFlags(ev[1], st, cudaEventRecordExternal));
         }
+        KF_TRY(record_raycast(v, st));
+        if (fork) KF_CK(cudaStreamWaitEvent(st, ev_join, 0));
+        if (profile) KF_CK(cudaEventRecordWithFlags(ev[2], st, cudaEventRecordExternal));
+        KF_TRY(record_pose(v, st));
+        if (profile) KF_CK(cudaEventRecordWithFlags(ev[3], st, cudaEventRecordExternal));
+        KF_TRY(record_fusion(v, st));
+        if (profile) KF_CK(cudaEventRecordWithFlags(ev[4], st, cudaEventRecordExternal));
+        return KF_OK;
+    }
+
+    kf_status record_raycast(const EngineView& v, cudaStream_t st) {
         // clear the wait record and the counters; the depth-range launch does it on the way
         if (has_range) {
             const int units_grid = int(std::min<long long>((tb.fuse_total + 255) / 256, sms * 4));
@@ -890,28 +901,29 @@ struct Engine {
         } else {
             KF_CK(cudaMemsetAsync(d_sync, 0, sizeof(GridSync) + sizeof(unsigned int) * kCounters, st));
         }
-        {
-            NvtxRange r("kf.raycast");
-            if (stages[1]) KF_CK(launch_raycast(v, shape.grid_ray, slot_fmt, st, ray_many));
-        }
-        if (fork) KF_CK(cudaStreamWaitEvent(st, ev_join, 0));
-        if (profile) KF_CK(cudaEventRecordWithFlags(ev[2], st, cudaEventRecordExternal));
-        {
-            NvtxRange r("kf.icp");
-            if (stages[2]) KF_CK(launch_icp(v, shape.grid_icp, st, cap == 1));
-        }
-        if (profile) KF_CK(cudaEventRecordWithFlags(ev[3], st, cudaEventRecordExternal));
+        NvtxRange r("kf.raycast");
+        if (stages[1]) KF_CK(launch_raycast(v, shape.grid_ray, slot_fmt, st, ray_many));
+        return KF_OK;
+    }
+
+    kf_status record_pose(const EngineView& v, cudaStream_t st) {
+        NvtxRange r("kf.icp");
+        if (stages[2]) KF_CK(launch_icp(v, shape.grid_icp, st, cap == 1));
+        return KF_OK;
+    }
+
+    kf_status record_fusion(const EngineView& v, cudaStream_t st) {
+        if (!stages[3]) return KF_OK;
         {
             NvtxRange r("kf.fusion");
-            if (stages[3]) KF_CK(launch_fuse(v, shape.grid_fuse, slot_fmt, st));
+            KF_CK(launch_fuse(v, shape.grid_fuse, slot_fmt, st));
         }
-        if (has_vis && stages[3]) {
+        if (has_vis) {
             // the visualization volumes (the reference's second grid), after the tracking fusion
             // and in the same stage time
             NvtxRange r("kf.fusion_vis");
             KF_CK(launch_fuse_vis(v, shape.grid_fuse, slot_fmt, st));
         }
-        if (profile) KF_CK(cudaEventRecordWithFlags(ev[4], st, cudaEventRecordExternal));
         return KF_OK;
     }
 
@@ -948,7 +960,7 @@ struct Engine {
         return KF_OK;
     }
 
-    kf_status enqueue(cudaStream_t st) {
+    kf_status upload_tables(cudaStream_t st) {
         if (tables_dirty) {
             KF_CK(cudaStreamSynchronize(st));
             KF_TRY(build_tables());
@@ -957,6 +969,51 @@ struct Engine {
             KF_CK(cudaMemcpyAsync(d_step, h_step, sizeof(StepDev) * cap, cudaMemcpyHostToDevice, st));
             step_dirty = false;
         }
+        return KF_OK;
+    }
+
+    // One step with its frames' copies.  copy(cs) puts them on stream cs; `src` is one of the frames
+    // (host memory unless `device`).
+    //
+    // A copy from pageable memory holds the calling thread until the frame is staged (some 50 us for
+    // 640x480), so the raycast, which needs only earlier frames, is launched before it, and the rest
+    // launch by launch while the raycast runs: 640x480 in 512^3 241 -> 219 us a frame, 320x240 in 128^3
+    // 142 -> 137.  Any other copy returns at once, and one graph launch costs less than seven: the whole
+    // step is one.  Profiled and counted steps, and steps on a stream that is being captured, too.
+    template <class Copy>
+    kf_status step(cudaStream_t st, const void* src, bool device, Copy&& copy) {
+        cudaStream_t cs = st;
+        if (!split_step(st, src, device)) {
+            KF_TRY(begin_inputs(st, &cs));
+            KF_TRY(copy(cs));
+            KF_TRY(end_inputs(cs));
+            return enqueue(st);
+        }
+        KF_TRY(upload_tables(st));
+        KF_TRY(begin_inputs(st, &cs));
+        const EngineView v = view();
+        KF_TRY(record_raycast(v, st));
+        KF_TRY(copy(cs));
+        KF_CK(launch_preprocess(v, shape.grid_pre, cs));
+        KF_TRY(end_inputs(cs));
+        KF_CK(cudaStreamWaitEvent(st, ev_input, 0));
+        KF_TRY(record_pose(v, st));
+        return record_fusion(v, st);
+    }
+
+    bool split_step(cudaStream_t st, const void* src, bool device) const {
+        if (device || profile || count_rays || !(stages[0] && stages[1])) return false;
+        cudaPointerAttributes a;
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaPointerGetAttributes(&a, src) != cudaSuccess || cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        return a.type == cudaMemoryTypeUnregistered && cs == cudaStreamCaptureStatusNone;
+    }
+
+    kf_status enqueue(cudaStream_t st) {
+        KF_TRY(upload_tables(st));
         if (use_graph) {
             if (graph_dirty || !gexec) KF_TRY(capture());
             if (use_graph) {
@@ -1294,12 +1351,11 @@ static kf_status session_enqueue(kf_session* s, const uint16_t* depth, int is_de
     want[s->slot] = StepDev{1, sl.frames == 0 ? 1 : 0};
     KF_TRY(s->eng->set_step(want, st));
     Engine& e = *s->eng;
-    cudaStream_t cs = st;
-    KF_TRY(e.begin_inputs(st, &cs));
-    KF_CK(cudaMemcpyAsync(const_cast<uint16_t*>(sl.d.raw), depth, bytes,
-                          is_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, cs));
-    KF_TRY(e.end_inputs(cs));
-    return e.enqueue(st);
+    return e.step(st, depth, is_dev != 0, [&](cudaStream_t cs) -> kf_status {
+        KF_CK(cudaMemcpyAsync(const_cast<uint16_t*>(sl.d.raw), depth, bytes,
+                              is_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, cs));
+        return KF_OK;
+    });
 }
 
 kf_status kf_process_frame(kf_session* s, const uint16_t* depth, int is_device_ptr, void* stream, float pose_out[16]) {
@@ -2041,16 +2097,17 @@ kf_status kf_batch_step(kf_batch* b, const uint16_t* const* depth, int is_device
     }
     KF_TRY(b->eng.set_step(want, st));
     KF_TRY(tuner_before_step(b->eng));
-    cudaStream_t cs = st;
-    KF_TRY(b->eng.begin_inputs(st, &cs));
-    for (int i = 0; i < b->n; ++i) {
-        if (!depth[i]) continue;
-        Slot& sl = b->eng.slots[i];
-        KF_CK(cudaMemcpyAsync(const_cast<uint16_t*>(sl.d.raw), depth[i], size_t(sl.cfg.width) * sl.cfg.height * 2,
-                              is_device_ptr ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, cs));
-    }
-    KF_TRY(b->eng.end_inputs(cs));
-    KF_TRY(b->eng.enqueue(st));
+    const uint16_t* first = nullptr;
+    for (int i = 0; i < b->n && !first; ++i) first = depth[i];
+    KF_TRY(b->eng.step(st, first, is_device_ptr != 0 || !first, [&](cudaStream_t cs) -> kf_status {
+        for (int i = 0; i < b->n; ++i) {
+            if (!depth[i]) continue;
+            Slot& sl = b->eng.slots[i];
+            KF_CK(cudaMemcpyAsync(const_cast<uint16_t*>(sl.d.raw), depth[i], size_t(sl.cfg.width) * sl.cfg.height * 2,
+                                  is_device_ptr ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, cs));
+        }
+        return KF_OK;
+    }));
     KF_TRY(b->eng.fetch(st));
     KF_CK(cudaStreamSynchronize(st));
     kf_status r = b->eng.collect(want);

@@ -290,3 +290,40 @@ def test_compute_pose_equals_the_session(kf, cuda, w, h, levels, side):
         if st == 0:
             np.testing.assert_array_equal(p.view(np.int32), np.asarray(pose, np.float32).view(np.int32))
     s.close()
+
+
+@pytest.mark.parametrize("w,h,n,vis", [(32, 24, 64, 0), (164, 124, 200, 48), (640, 480, 256, 0)])
+def test_frames_from_any_memory_agree(kf, cuda, w, h, n, vis):
+    """Frames from pageable memory (the raycast is launched before their copy), pinned memory and the
+    device give the same poses and volumes, blocking and two in flight, in a session, a profiled
+    session and a batch; the kinds may follow one another in one session."""
+    from kfb200 import synth
+    cfg = kf.config_small(width=w, height=h, fx=262.5 * w / 320, fy=262.5 * w / 320, cx=w / 2 - 0.5, cy=h / 2 - 0.5,
+                          volume_n=n, mu=max(0.03, 6.0 / n), vis_volume_n=vis, vis_volume_width=5.0, vis_mu=0.2)
+    imgs, _ = synth.sequence(cfg, 5, seed=6, kind=synth.LOOP)
+    pinned = [cuda.from_numpy(i.copy()).pin_memory() for i in imgs]
+    kinds = {"pageable": list(imgs), "pinned": [p.numpy() for p in pinned], "device": [dev(cuda, i) for i in imgs]}
+    kinds["mixed"] = [kinds[("pageable", "device", "pinned")[i % 3]][i] for i in range(5)]
+    wants = {}
+    for name, frames in kinds.items():
+        runs = ["blocking", "profiled", "flying"] + (["batch"] if name in ("pageable", "pinned") else [])
+        for how in runs:
+            b = kf.Batch([cfg, cfg]) if how == "batch" else None
+            s = b.session(1) if b else kf.KinectFusion(cfg)
+            if how == "profiled":
+                s.set_profiling(True)
+            poses = []
+            if b:
+                poses = [b.step([f, f])[1][1] for f in frames]
+            elif how == "flying":
+                for i, f in enumerate(frames):
+                    s.submit_frame(f)
+                    if i:
+                        poses.append(s.wait_frame()[1])
+                poses.append(s.wait_frame()[1])
+            else:
+                poses = [s.process_frame(f)[1] for f in frames]
+            got = [np.asarray(poses, np.float32).reshape(5, 16), *s.tsdf(), *(s.vis_tsdf() if vis else ())]
+            for a, c in zip(wants.setdefault("batch" if b else "alone", got), got):
+                np.testing.assert_array_equal(a, c, err_msg=name + " " + how)
+            (b or s).close()
