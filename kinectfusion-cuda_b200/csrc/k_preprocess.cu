@@ -215,15 +215,31 @@ __global__ void convert_kernel(const uint16_t* raw, float* out, int w, int h, fl
     out[size_t(j) * w + io] = d;
 }
 
-__global__ void bilateral_kernel(const float* in, float* out, int w, int h, float inv_ss, float inv_sr, int R) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+// A block filters 32 x 8 pixels from shared memory, where a pixel's taps cost a load each; read through
+// the cache with clamped indices every tap cost a dozen instructions more.  kR as in preprocess_tile.
+// 640x480, radius 3: 15.8 -> 9.1 us, most of it now the 49 exponentials.
+constexpr int kBilW = 32, kBilH = 8;
+
+template <int kR>
+__global__ void __launch_bounds__(kBilW * kBilH) bilateral_kernel(const float* in, float* out, int w, int h, float inv_ss,
+                                                                  float inv_sr, int radius) {
+    __shared__ float reg[(kBilW + 2 * kMaxBilateralRadius) * (kBilH + 2 * kMaxBilateralRadius)];
+    const int R = kR ? kR : radius, pitch = kBilW + 2 * R;
+    const int across = (w + kBilW - 1) / kBilW, x0 = blockIdx.x % across * kBilW, y0 = blockIdx.x / across * kBilH;
+    for (int idx = threadIdx.x; idx < pitch * (kBilH + 2 * R); idx += kBilW * kBilH) {
+        const int x = min(max(x0 - R + idx % pitch, 0), w - 1), y = min(max(y0 - R + idx / pitch, 0), h - 1);
+        reg[idx] = __ldg(in + size_t(y) * w + x);
+    }
+    __syncthreads();
+    const int lx = threadIdx.x % kBilW, ly = threadIdx.x / kBilW, i = x0 + lx, j = y0 + ly;
     if (i >= w || j >= h) return;
-    out[size_t(j) * w + i] = bilateral_core(
-        [in, w, h, i, j](int x, int y) {
-            const int xx = min(max(i + x, 0), w - 1), yy = min(max(j + y, 0), h - 1);
-            return __ldg(in + size_t(yy) * w + xx);
-        },
-        R, inv_ss, inv_sr);
+    const float* c = reg + (ly + R) * pitch + lx + R;
+    float d;
+    if constexpr (kR > 0)
+        d = bilateral_fixed<kR>([c](int x, int y) { return c[y * (kBilW + 2 * kR) + x]; }, inv_ss, inv_sr);
+    else
+        d = bilateral_core([c, pitch](int x, int y) { return c[y * pitch + x]; }, R, inv_ss, inv_sr);
+    out[size_t(j) * w + i] = d;
 }
 
 __global__ void downsample_kernel(const float* in, float* out, int wo, int ho, float thr) {
@@ -255,7 +271,11 @@ cudaError_t stage_convert(const uint16_t* raw, float* out, int w, int h, float s
     return cudaGetLastError();
 }
 cudaError_t stage_bilateral(const float* in, float* out, int w, int h, float ss, float sr, int r, cudaStream_t st) {
-    bilateral_kernel<<<grid2(w, h), dim3(16, 16), 0, st>>>(in, out, w, h, 1.0f / (ss * ss), 1.0f / (sr * sr), r);
+    const unsigned int grid = unsigned((w + kBilW - 1) / kBilW) * unsigned((h + kBilH - 1) / kBilH);
+    const float inv_ss = 1.0f / (ss * ss), inv_sr = 1.0f / (sr * sr);
+    if (r == 2) bilateral_kernel<2><<<grid, kBilW * kBilH, 0, st>>>(in, out, w, h, inv_ss, inv_sr, r);
+    else if (r == 3) bilateral_kernel<3><<<grid, kBilW * kBilH, 0, st>>>(in, out, w, h, inv_ss, inv_sr, r);
+    else bilateral_kernel<0><<<grid, kBilW * kBilH, 0, st>>>(in, out, w, h, inv_ss, inv_sr, r);
     return cudaGetLastError();
 }
 cudaError_t stage_down_sample(const float* in, float* out, int wo, int ho, float sr, cudaStream_t st) {

@@ -327,3 +327,17 @@ def test_frames_from_any_memory_agree(kf, cuda, w, h, n, vis):
             for a, c in zip(wants.setdefault("batch" if b else "alone", got), got):
                 np.testing.assert_array_equal(a, c, err_msg=name + " " + how)
             (b or s).close()
+
+
+@pytest.mark.parametrize("w,h,radius", [(1, 1, 3), (31, 7, 0), (33, 9, 2), (64, 8, 3), (161, 119, 1), (97, 65, 7),
+                                        (161, 119, 3)])
+def test_bilateral_shapes(kf, orc, cuda, w, h, radius):
+    """Blocks that overhang the image and halos that clamp, at every kind of radius; a filtered depth
+    is a mean of values up to 6 m with weights of the fast exponential (2e-6 relative), so it agrees
+    with the FP64 oracle to 2e-5 m."""
+    rng = np.random.default_rng(w * 31 + h)
+    d = (rng.uniform(0.5, 6.0) + 0.05 * rng.standard_normal((h, w))).astype(np.float32)
+    out = cuda.zeros((h, w), device="cuda")
+    kf.kernel.applyBilateralFilter(dev(cuda, d), out, 4.0, 0.25, radius)
+    want = orc.bilateral(d, 4.0, 0.25, radius, prec=1)
+    np.testing.assert_allclose(out.cpu().numpy(), want, atol=2e-5, rtol=0)
