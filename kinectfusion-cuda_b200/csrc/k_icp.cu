@@ -283,37 +283,6 @@ __device__ __forceinline__ void m3d_vec(const double* m, const double* v, double
     for (int r = 0; r < 3; ++r) o[r] = m[r] * v[0] + m[3 + r] * v[1] + m[6 + r] * v[2];
 }
 
-// the 24 floats phase A of the next pass reads for a session at level Lv: the estimate
-// (R, t), M = K_l * R_prev^T and t_prev
-__device__ void publish_mats(float* m, const double* R, const double* t, const double* Rp, const float* tpf,
-                             const LevelDev& Lv) {
-    for (int q = 0; q < 9; ++q) m[q] = float(R[q]);
-    for (int q = 0; q < 3; ++q) m[9 + q] = float(t[q]);
-    // K = [fx 0 cx; 0 fy cy; 0 0 1];  M = K * Rp^T;  (Rp^T)(r, c) = Rp(c, r) = Rp[r * 3 + c]
-    for (int col = 0; col < 3; ++col) {
-        // column col of Rp^T = row col of Rp = (Rp[col], Rp[3 + col], Rp[6 + col])
-        const double a0 = Rp[col], a1 = Rp[3 + col], a2 = Rp[6 + col];
-        m[12 + col * 3 + 0] = float(double(Lv.fx) * a0 + double(Lv.cx) * a2);
-        m[12 + col * 3 + 1] = float(double(Lv.fy) * a1 + double(Lv.cy) * a2);
-        m[12 + col * 3 + 2] = float(a2);
-    }
-    for (int q = 0; q < 3; ++q) m[21 + q] = tpf[q];
-}
-
-// first ICP level with iterations at or below `from`
-__device__ __forceinline__ int next_level(const SessionDev* S, int from) {
-    int l = from;
-    while (l >= 0 && S->iters[l] <= 0) --l;
-    return l;
-}
-
-// schedule entry of a session: the level of its next pass and that level's tiles
-__device__ __forceinline__ int4 sched_entry(const EngineView& v, int s, int level) {
-    if (level < 0) return make_int4(-1, 0, 0, 0);
-    const IcpRange rg = v.iranges[level * v.tb->S + s];
-    return make_int4(level, rg.begin, rg.end - rg.begin, 0);
-}
-
 // Where a session's ICP iteration state lives: in the session's pose block and the engine's
 // schedule and matrix arrays (one owner block updates them and a grid barrier publishes
 // them), or in a block's shared memory (every block updates its own copy, identically).
@@ -347,28 +316,71 @@ __device__ __forceinline__ IcpStateRef local_state(IcpLocal& L) {
     return IcpStateRef{L.R, L.t, &L.it, L.iters, &L.level, &L.cont, &L.status, L.mats, &L.sched};
 }
 
-// phase 0 for one session (one thread); every slot gets a schedule entry
-__device__ void icp_begin(const EngineView& v, int s, const IcpStateRef& ref) {
+// phase 0 for one session (one thread); every slot gets a schedule entry.  Every block waits for it, and
+// icp_finish holds up the fusion: both read all they need into registers before their first store,
+// two round trips each, where a store through a pointer that could alias the next load made a chain
+// of some twenty: 640x480, one session 46.1 -> 42.0 us in the kernel (a frame of a stream 191 -> 187),
+// 24 sessions 272 -> 268.
+__device__ __forceinline__ void icp_begin(const EngineView& v, int s, const IcpStateRef& ref) {
     const SessionDev* S = &v.sess[s];
     const StepDev st = v.step[s];
+    const PoseDev* P = S->pose;
+    const int levels = S->L, slots = v.tb->S;
+    int iters[kMaxLevels];
+#pragma unroll
+    for (int l = 0; l < kMaxLevels; ++l) iters[l] = S->iters[l];
     if (!st.active) {   // empty or idle slot: its state is not touched
         *ref.sched = make_int4(-1, 0, 0, 0);
         return;
     }
-    const PoseDev* P = S->pose;
+    int level = -1;   // the first level with iterations, from the coarsest
+    if (!st.first) {
+#pragma unroll
+        for (int l = 0; l < kMaxLevels; ++l)
+            if (l < levels && iters[l] > 0) level = l;
+    }
+    const int at = max(level, 0);
+    double R[9], t[3];
+    float tpf[3];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) R[q] = P->Rp[q];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) { t[q] = P->tp[q]; tpf[q] = P->tpf[q]; }
+    const float fx = S->lv[at].fx, fy = S->lv[at].fy, cx = S->lv[at].cx, cy = S->lv[at].cy;
+    const IcpRange rg = v.iranges[at * slots + s];
+
     *ref.status = KF_OK;
+#pragma unroll
     for (int l = 0; l < kMaxLevels; ++l) ref.iters[l] = 0;
     *ref.it = 0;
-    int level = -1;
     if (!st.first) {
-        for (int q = 0; q < 9; ++q) ref.R[q] = P->Rp[q];
-        for (int q = 0; q < 3; ++q) ref.t[q] = P->tp[q];
-        level = next_level(S, S->L - 1);
-        if (level >= 0) publish_mats(ref.mats, P->Rp, P->tp, P->Rp, P->tpf, S->lv[level]);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) ref.R[q] = R[q];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) ref.t[q] = t[q];
+    }
+    if (level >= 0) {
+        // the 24 floats phase A reads: the estimate (R, t), M = K_l * R_prev^T and t_prev, with
+        // K = [fx 0 cx; 0 fy cy; 0 0 1] and (Rp^T)(r, c) = Rp(c, r) = Rp[r * 3 + c]
+        float* m = ref.mats;
+#pragma unroll
+        for (int q = 0; q < 9; ++q) m[q] = float(R[q]);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) m[9 + q] = float(t[q]);
+#pragma unroll
+        for (int col = 0; col < 3; ++col) {
+            // column col of Rp^T = row col of Rp = (Rp[col], Rp[3 + col], Rp[6 + col])
+            const double a0 = R[col], a1 = R[3 + col], a2 = R[6 + col];
+            m[12 + col * 3 + 0] = float(double(fx) * a0 + double(cx) * a2);
+            m[12 + col * 3 + 1] = float(double(fy) * a1 + double(cy) * a2);
+            m[12 + col * 3 + 2] = float(a2);
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) m[21 + q] = tpf[q];
     }
     *ref.level = level;
     *ref.cont = level >= 0 ? 1 : 0;
-    *ref.sched = sched_entry(v, s, level);
+    *ref.sched = level >= 0 ? make_int4(level, rg.begin, rg.end - rg.begin, 0) : make_int4(-1, 0, 0, 0);
     // no fence here: thread 0 writes all of this, and the grid barrier that follows fences
     // thread 0's writes before it arrives
 }
@@ -387,9 +399,9 @@ __device__ void icp_solve(const EngineView& v, int s, int level, int begin, int 
     const int tid = threadIdx.x, lane = tid & 31;
     // warp 0 fetches everything the update needs while the block sums the tiles
     double R0[9], t0[3], Rp[9];
-    int it0 = 0, done0 = 0, S_cap = 0, siters[kMaxLevels];
-    float stop_a = 0.f, stop_d = 0.f, tpf[3], lfx[kMaxLevels], lfy[kMaxLevels], lcx[kMaxLevels], lcy[kMaxLevels];
-    IcpRange rng[kMaxLevels];
+    int it0 = 0, done0 = 0, cap = 0, below = -1;
+    float stop_a = 0.f, stop_d = 0.f, tpf[3], kfx[2], kfy[2], kcx[2], kcy[2];   // this level's and the next's
+    IcpRange rng[2];
     if (tid < 32) {
 #pragma unroll
         // the state was written by this block's thread 0 (ordered by the block barriers)
@@ -398,16 +410,21 @@ __device__ void icp_solve(const EngineView& v, int s, int level, int begin, int 
         for (int q = 0; q < 3; ++q) { t0[q] = ref.t[q]; tpf[q] = ldcg(&P->tpf[q]); }
         it0 = *ref.it;
         done0 = ref.iters[level];
-        S_cap = v.tb->S;
         stop_a = S->stop_a;
         stop_d = S->stop_d;
 #pragma unroll
         for (int l = 0; l < kMaxLevels; ++l) {
-            siters[l] = S->iters[l];
-            lfx[l] = S->lv[l].fx; lfy[l] = S->lv[l].fy; lcx[l] = S->lv[l].cx; lcy[l] = S->lv[l].cy;
+            const int n = S->iters[l];
+            if (l == level) cap = n;
+            if (l < level && n > 0) below = l;   // the next level with iterations
         }
+        const int S_cap = v.tb->S;
 #pragma unroll
-        for (int l = 0; l < kMaxLevels; ++l) rng[l] = v.iranges[l * S_cap + s];
+        for (int k = 0; k < 2; ++k) {
+            const int l = k ? max(below, 0) : level;
+            kfx[k] = S->lv[l].fx; kfy[k] = S->lv[l].fy; kcx[k] = S->lv[l].cx; kcy[k] = S->lv[l].cy;
+            rng[k] = v.iranges[l * S_cap + s];
+        }
     }
     // partial pairs as float4 (two entries each): thread (g, q) adds, in FP64 and in tile
     // order, entries 2q and 2q + 1 of tiles g, g + 18, g + 36, ...; 9 tiles' loads in flight,
@@ -496,12 +513,12 @@ __device__ void icp_solve(const EngineView& v, int s, int level, int begin, int 
                              (t0[2] - t1[2]) * (t0[2] - t1[2]));
     int it = it0 + 1;
     int lvl = level;
-    if ((ang < double(stop_a) && dist < double(stop_d)) || it >= siters[level]) {
-        lvl = level - 1;   // next level with iterations (next_level)
-        while (lvl >= 0 && siters[lvl] <= 0) --lvl;
+    if ((ang < double(stop_a) && dist < double(stop_d)) || it >= cap) {
+        lvl = below;
         it = 0;
     }
     if (lane != 0) return;
+    const bool same = lvl == level;
 #pragma unroll
     for (int r = 0; r < 9; ++r) ref.R[r] = R1[r];
 #pragma unroll
@@ -511,22 +528,25 @@ __device__ void icp_solve(const EngineView& v, int s, int level, int begin, int 
     *ref.level = lvl;
     *ref.cont = lvl >= 0 ? 1 : 0;
     if (lvl >= 0) {
+        const float fx = same ? kfx[0] : kfx[1], fy = same ? kfy[0] : kfy[1], ox = same ? kcx[0] : kcx[1],
+                    oy = same ? kcy[0] : kcy[1];
+        const IcpRange next = same ? rng[0] : rng[1];
         float* m = ref.mats;
 #pragma unroll
         for (int r = 0; r < 9; ++r) m[r] = float(R1[r]);
 #pragma unroll
         for (int r = 0; r < 3; ++r) m[9 + r] = float(t1[r]);
-        // M = K_l * Rp^T (as publish_mats)
+        // M = K_l * Rp^T (as icp_begin)
 #pragma unroll
         for (int col = 0; col < 3; ++col) {
             const double b0 = Rp[col], b1 = Rp[3 + col], b2 = Rp[6 + col];
-            m[12 + col * 3 + 0] = float(double(lfx[lvl]) * b0 + double(lcx[lvl]) * b2);
-            m[12 + col * 3 + 1] = float(double(lfy[lvl]) * b1 + double(lcy[lvl]) * b2);
+            m[12 + col * 3 + 0] = float(double(fx) * b0 + double(ox) * b2);
+            m[12 + col * 3 + 1] = float(double(fy) * b1 + double(oy) * b2);
             m[12 + col * 3 + 2] = float(b2);
         }
 #pragma unroll
         for (int r = 0; r < 3; ++r) m[21 + r] = tpf[r];
-        *ref.sched = make_int4(lvl, rng[lvl].begin, rng[lvl].end - rng[lvl].begin, 0);
+        *ref.sched = make_int4(lvl, next.begin, next.end - next.begin, 0);
     } else {
         *ref.sched = make_int4(-1, 0, 0, 0);
     }
@@ -534,38 +554,72 @@ __device__ void icp_solve(const EngineView& v, int s, int level, int begin, int 
 }
 
 // phase C for one session (one thread): the frame's pose becomes the previous pose; the
-// inverse feeds fusion; the result block goes to the host.
-__device__ void icp_finish(const SessionDev* S, const StepDev st, OutDev* out, FuseCtx* fctx, FuseCtx* vis_fctx) {
-    if (!st.active) return;
+// inverse feeds fusion; the result block goes to the host.  loc: the block-local state, which goes
+// back to the session's pose block, or null when that holds the state already.
+__device__ __forceinline__ void icp_finish(const SessionDev* S, const StepDev st, OutDev* out, FuseCtx* fctx,
+                                           FuseCtx* vis_fctx, const IcpLocal* loc) {
     PoseDev* P = S->pose;
-    const bool ok = P->status == KF_OK;
-    if (ok && !st.first) {
-        for (int q = 0; q < 9; ++q) P->Rp[q] = P->R[q];
-        for (int q = 0; q < 3; ++q) P->tp[q] = P->t[q];
+    if (!st.active) return;
+    double R[9], t[3], Rp[9], tp[3];
+    int iters[kMaxLevels];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) { R[q] = loc ? loc->R[q] : P->R[q]; Rp[q] = P->Rp[q]; }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) { t[q] = loc ? loc->t[q] : P->t[q]; tp[q] = P->tp[q]; }
+#pragma unroll
+    for (int l = 0; l < kMaxLevels; ++l) iters[l] = loc ? loc->iters[l] : P->iters[l];
+    const int status = loc ? loc->status : P->status, frame = P->frame + 1;
+    const bool ok = status == KF_OK;
+    if (loc) {
+        if (!st.first) {   // a first frame has no estimate (fusion only)
+#pragma unroll
+            for (int q = 0; q < 9; ++q) P->R[q] = R[q];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) P->t[q] = t[q];
+        }
+#pragma unroll
+        for (int l = 0; l < kMaxLevels; ++l) P->iters[l] = iters[l];
+        P->it = loc->it;
+        P->level = loc->level;
+        P->cont = loc->cont;
+        P->status = status;
     }
-    for (int q = 0; q < 9; ++q) P->Rpf[q] = float(P->Rp[q]);
-    for (int q = 0; q < 3; ++q) P->tpf[q] = float(P->tp[q]);
+    if (ok && !st.first) {
+#pragma unroll
+        for (int q = 0; q < 9; ++q) P->Rp[q] = Rp[q] = R[q];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) P->tp[q] = tp[q] = t[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 9; ++q) P->Rpf[q] = float(Rp[q]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) P->tpf[q] = float(tp[q]);
     // inverse, for the frame's fusion: R^T, -R^T t
-    float iR[9], it[3];
-    for (int c = 0; c < 3; ++c)
-        for (int r = 0; r < 3; ++r) iR[c * 3 + r] = float(P->Rp[r * 3 + c]);
-    for (int r = 0; r < 3; ++r)
-        it[r] = float(-(P->Rp[r * 3 + 0] * P->tp[0] + P->Rp[r * 3 + 1] * P->tp[1] + P->Rp[r * 3 + 2] * P->tp[2]));
+    float it[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) it[r] = float(-(Rp[r * 3 + 0] * tp[0] + Rp[r * 3 + 1] * tp[1] + Rp[r * 3 + 2] * tp[2]));
     for (FuseCtx* f : {fctx, vis_fctx}) {
-        for (int q = 0; q < 9; ++q) f->iR[q] = iR[q];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int r = 0; r < 3; ++r) f->iR[c * 3 + r] = float(Rp[r * 3 + c]);
+#pragma unroll
         for (int q = 0; q < 3; ++q) f->it[q] = it[q];
         f->ok = ok ? 1 : 0;
     }
-    P->frame += 1;
-    for (int q = 0; q < 16; ++q) out->pose[q] = 0.f;
-    for (int c = 0; c < 3; ++c)
-        for (int r = 0; r < 3; ++r) out->pose[c * 4 + r] = P->Rpf[c * 3 + r];
-    for (int r = 0; r < 3; ++r) out->pose[12 + r] = P->tpf[r];
+    P->frame = frame;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+        for (int r = 0; r < 3; ++r) out->pose[c * 4 + r] = float(Rp[c * 3 + r]);
+        out->pose[c * 4 + 3] = 0.f;
+        out->pose[12 + c] = float(tp[c]);
+    }
     out->pose[15] = 1.f;
-    for (int l = 0; l < kMaxLevels; ++l) out->iters[l] = P->iters[l];
-    out->status = P->status;
-    out->frame = P->frame;
-    __threadfence();
+#pragma unroll
+    for (int l = 0; l < kMaxLevels; ++l) out->iters[l] = iters[l];
+    out->status = status;
+    out->frame = frame;
 }
 
 // In-place inclusive scan of a[0..n) in shared memory by the whole block (n <= 1024).
@@ -624,19 +678,6 @@ __device__ __forceinline__ void icp_group(const EngineView& v, int s, int lvl, i
                                          [&](const float (&a)[6], float b) { accumulate_products(acc, a, b); });
     }
     block_reduce_store(acc, red, out);
-}
-
-// thread 0: the block-local state goes back to the session's pose block
-__device__ void store_local_state(PoseDev* P, const IcpLocal& L, bool first) {
-    if (!first) {   // a first frame has no estimate (fusion only)
-        for (int q = 0; q < 9; ++q) P->R[q] = L.R[q];
-        for (int q = 0; q < 3; ++q) P->t[q] = L.t[q];
-    }
-    for (int l = 0; l < kMaxLevels; ++l) P->iters[l] = L.iters[l];
-    P->it = L.it;
-    P->level = L.level;
-    P->cont = L.cont;
-    P->status = L.status;
 }
 
 // A batch's launch holds two blocks per SM (128 registers; the solve, run once per session
@@ -729,13 +770,10 @@ __global__ void __launch_bounds__(kIcpThreads, local ? 1 : 2) icp_kernel(EngineV
 
     if constexpr (local) {
         // block 0 stores the state the rest of the frame and the host read
-        if (blockIdx.x == 0 && tid == 0 && v.step[0].active) {
-            store_local_state(v.sess[0].pose, loc, v.step[0].first != 0);
-            icp_finish(&v.sess[0], v.step[0], v.out, v.fctx, v.vis_fctx);
-        }
+        if (blockIdx.x == 0 && tid == 0) icp_finish(&v.sess[0], v.step[0], v.out, v.fctx, v.vis_fctx, &loc);
     } else {
         for (int s = blockIdx.x; s < S_cap; s += gridDim.x)
-            if (tid == 0) icp_finish(&v.sess[s], v.step[s], v.out + s, v.fctx + s, v.vis_fctx + s);
+            if (tid == 0) icp_finish(&v.sess[s], v.step[s], v.out + s, v.fctx + s, v.vis_fctx + s, nullptr);
     }
 }
 
