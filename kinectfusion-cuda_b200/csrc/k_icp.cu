@@ -652,29 +652,36 @@ __device__ void block_inclusive_scan(int* a, int n, int* warp_tot) {
 constexpr int kIcpMaxSessionsSmem = 1024;
 constexpr int kIcpPixelsPerStep = 4;   // pixels a thread carries through one pipelined step
 
+// What phase A needs of one session-level.  tile: pixels of every tile but the last (0: look the tiles up).
+struct IcpLevel {
+    const float4 *vm, *tv, *tn;
+    uint8_t* mask;
+    int w, h, icw, total, tile;
+    float dist, cos_th;
+};
+
+__device__ __forceinline__ IcpLevel icp_level(const SessionDev* S, int lvl, int tile) {
+    const LevelDev& Lv = S->lv[lvl];
+    return IcpLevel{S->vmap[lvl], S->pv[lvl], S->pn[lvl], S->mask[lvl], Lv.w, Lv.h, Lv.icw, Lv.icw * Lv.ich, tile,
+                    S->dist_th, S->angle_cos};
+}
+
 // Phase A of one group: tiles g, g + G, ... of a session at one level, accumulated by the whole
 // block in tile order (each thread its pixels p0 + tid, p0 + tid + 256, ... of each tile), then
 // reduced to one compensated partial at `out`.  The partial depends on the group's tiles only,
 // not on which block or launch computes it.
-__device__ __forceinline__ void icp_group(const EngineView& v, int s, int lvl, int tile0, int ntiles, int g, int G,
+__device__ __forceinline__ void icp_group(const EngineView& v, const IcpLevel& L, int tile0, int ntiles, int g, int G,
                                           const float* mats, float* red, float* out) {
     float acc[32];
 #pragma unroll
     for (int q = 0; q < 32; ++q) acc[q] = 0.f;
-    const SessionDev* S = &v.sess[s];
-    const LevelDev& Lv = S->lv[lvl];
-    const float4* vm = S->vmap[lvl];
-    const float4* tv = S->pv[lvl];
-    const float4* tn = S->pn[lvl];
-    uint8_t* mask = S->mask[lvl];
-    const float dist = S->dist_th, ang = S->angle_cos;
     const IcpMats m{mats, mats + 9, mats + 12, mats + 21};
     for (int j = g; j < ntiles; j += G) {
-        const IcpTile T = v.itiles[tile0 + j];
+        const IcpTile T = L.tile ? IcpTile{0, j * L.tile, min(L.tile, L.total - j * L.tile)} : v.itiles[tile0 + j];
         const int pend = T.p0 + T.np;
 #pragma unroll 1
         for (int p = T.p0 + threadIdx.x; p < pend; p += kIcpPixelsPerStep * kIcpThreads)
-            icp_multi<kIcpPixelsPerStep>(vm, tv, tn, Lv.w, Lv.h, Lv.icw, p, pend, m, dist, ang, mask,
+            icp_multi<kIcpPixelsPerStep>(L.vm, L.tv, L.tn, L.w, L.h, L.icw, p, pend, m, L.dist, L.cos_th, L.mask,
                                          [&](const float (&a)[6], float b) { accumulate_products(acc, a, b); });
     }
     block_reduce_store(acc, red, out);
@@ -694,6 +701,7 @@ __global__ void __launch_bounds__(kIcpThreads, local ? 1 : 2) icp_kernel(EngineV
     __shared__ int s_cnt[kIcpMaxSessionsSmem];       // tiles of session s at its level
     __shared__ int s_wtot[kIcpThreads / 32];
     __shared__ IcpLocal loc;
+    __shared__ IcpLevel levels[kMaxLevels];   // local only
     const int tid = threadIdx.x;
     const unsigned int nb = gridDim.x;
     unsigned int epoch = 0;
@@ -705,8 +713,16 @@ __global__ void __launch_bounds__(kIcpThreads, local ? 1 : 2) icp_kernel(EngineV
     // partials while another still sums this pass's; a block two passes on has passed a
     // barrier that every block reaches only after its solve.
 
+    // Its levels stay in shared memory for the whole launch: the grid barrier's acquire empties the L1,
+    // so every pass had waited for them again before its first vertex (kernel 42.0 -> 41.2 us, six
+    // frames of a stream 1105 -> 1097).
     if (local) {
         if (tid == 0) icp_begin(v, 0, local_state(loc));
+        const int l = tid - 32;
+        if (l >= 0 && l < kMaxLevels) {
+            const IcpRange rg = v.iranges[l * S_cap];
+            levels[l] = icp_level(v.sess, l, rg.begin < rg.end ? v.itiles[rg.begin].np : 1);
+        }
         __syncthreads();
     } else {
         for (int s = blockIdx.x; s < S_cap; s += gridDim.x)
@@ -747,8 +763,9 @@ __global__ void __launch_bounds__(kIcpThreads, local ? 1 : 2) icp_kernel(EngineV
                     if (tid < 24) mats[tid] = local ? loc.mats[tid] : ldcg(v.icp_mats + size_t(s) * 24 + tid);
                     __syncthreads();
                 }
-                icp_group(v, s, lvl, s_beg[s], s_cnt[s], g, kIcpGroups, mats, red,
-                                 parts + size_t(s_beg[s] + g) * kIcpPartialStride);
+                float* const out = parts + size_t(s_beg[s] + g) * kIcpPartialStride;
+                if constexpr (local) icp_group(v, levels[lvl], s_beg[s], s_cnt[s], g, kIcpGroups, mats, red, out);
+                else icp_group(v, icp_level(&v.sess[s], lvl, 0), s_beg[s], s_cnt[s], g, kIcpGroups, mats, red, out);
             }
         }
         if (!grid_barrier(v.sync, nb, epoch)) return;
