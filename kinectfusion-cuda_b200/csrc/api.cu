@@ -1880,7 +1880,7 @@ kf_status kf_raycast(const kf_volume* vol, const float pose[16], const float inv
         !(vol->mu * step_small > max_depth * 1e-6f))
         return KF_ERR_ARG;
     cudaStream_t st = as_stream(stream);
-    const bool build = stage_raycast_builds_bounds(vol, w, h);
+    const bool build = stage_raycast_builds_bounds(vol, w, h, min_depth);
     const int cap = ray_queue_entries(w, h, build);
     Scratch scratch;
     raycast_scratch(scratch, build ? vol->n : 0, w, h, cap, st);

@@ -126,7 +126,7 @@ __device__ __forceinline__ void range_bricks(const RangeView& r, bool on, int bx
             // 0.1 px covers the rounding of the rays' and the corners' projections
             umin -= 0.1f; vmin -= 0.1f; umax += 0.1f; vmax += 0.1f;
             if (!(zmin > 1e-3f)) {   // reaches the camera plane: no image
-                range_add(r.range + 2 * r.rgw * r.rgh, 0.0f, zmax);
+                range_add(r.range + 2 * r.rgw * r.rgh, 0.0f, fmaxf(zmax, 0.0f));
             } else if (umax >= 0.f && vmax >= 0.f && umin <= float(r.w) && vmin <= float(r.h)) {
                 x0 = int(fmaxf(umin, 0.f)) / kRangeTile;
                 x1 = min(int(fminf(umax, float(r.w))) / kRangeTile, r.rgw - 1);
@@ -1175,8 +1175,11 @@ __global__ void raycast_stage_kernel(SessionDev S, RayStage rs, int w, int h) {
 // (f16 202 / 148).  The line lies between the two images.
 constexpr long long kBoundsRays = 160000;
 
-bool stage_raycast_builds_bounds(const kf_volume* vol, int w, int h) {
-    return (long long)w * h >= kBoundsRays && reinterpret_cast<uintptr_t>(vol->f) % 16 == 0;   // vector reads
+// A depth range that begins behind the camera has no bounds: the frustum's planes and the depth ranges
+// hold for samples ahead of it.
+bool stage_raycast_builds_bounds(const kf_volume* vol, int w, int h, float min_d) {
+    return min_d >= 0.0f && (long long)w * h >= kBoundsRays &&
+           reinterpret_cast<uintptr_t>(vol->f) % 16 == 0;   // vector reads
 }
 
 // Without bounds a lane's budget is short for small images, whose few warps leave the GPU idle
@@ -1284,7 +1287,7 @@ cudaError_t stage_raycast(const kf_volume* vol, const float* pose, const float* 
             if (!std::isfinite(rs.inv[q])) rs.has_inv = 0;
         }
     }
-    const bool build = !bounds && stage_raycast_builds_bounds(vol, w, h);
+    const bool build = !bounds && stage_raycast_builds_bounds(vol, w, h, min_d);
     if (vol->format == KF_TSDF_F16U16) return launch_stage<__half>(S, rs, w, h, build, scratch, longq_cap, st);
     return launch_stage<float>(S, rs, w, h, build, scratch, longq_cap, st);
 }

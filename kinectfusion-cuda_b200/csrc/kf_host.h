@@ -154,7 +154,7 @@ cudaError_t stage_normal(const float4* v, float4* n, int w, int h, cudaStream_t 
 // bounds (optional): a session whose brick bounds the march may use to skip.  scratch:
 // stage_raycast_scratch bytes of device memory with room for longq_cap long rays (n: the volume's
 // size when the call builds bounds, else 0), or null to march every ray in its own thread.
-bool stage_raycast_builds_bounds(const kf_volume* vol, int w, int h);
+bool stage_raycast_builds_bounds(const kf_volume* vol, int w, int h, float min_d);
 int stage_raycast_queue(int w, int h, bool bounds, long long share);   // share: a session's entries
 size_t stage_raycast_scratch(int n, int w, int h, int longq_cap);
 cudaError_t stage_raycast(const kf_volume* vol, const float* pose, const float* ik, float4* vtx, float4* nrm, int w,

@@ -341,3 +341,28 @@ def test_bilateral_shapes(kf, orc, cuda, w, h, radius):
     kf.kernel.applyBilateralFilter(dev(cuda, d), out, 4.0, 0.25, radius)
     want = orc.bilateral(d, 4.0, 0.25, radius, prec=1)
     np.testing.assert_allclose(out.cpu().numpy(), want, atol=2e-5, rtol=0)
+
+
+@pytest.mark.parametrize("n,w,h,fmt", [(136, 500, 330, 0), (200, 500, 331, 0), (200, 501, 330, 1)])
+@pytest.mark.parametrize("depths", [(-1.5, 6.0), (-0.9, -0.05)])
+def test_raycast_behind_the_camera(kf, cuda, n, w, h, fmt, depths):
+    """A depth range that begins (or lies) behind the camera is a march like any other: from the middle
+    of a volume with a sphere ahead and one behind, the maps of the march of every sample, bit for
+    bit, and hits on both sides."""
+    width, mu = 2.0, max(0.02, 3.0 / n)
+    x = (cuda.arange(n, device="cuda", dtype=cuda.float32) + 0.5) * (width / n) - width / 2
+    z, y, x = cuda.meshgrid(x, x, x, indexing="ij")
+    d = [cuda.sqrt(x * x + y * y + (z - c) ** 2) - 0.25 for c in (0.6, -0.6)]
+    f = cuda.clamp(cuda.minimum(*d) / mu, -1.0, 1.0)
+    f = (f.half() if fmt else f).contiguous()
+    vol = kf.kernel.volume(f, cuda.zeros_like(f), width, mu, fmt=fmt)
+    ik = np.linalg.inv(np.array([[300, 0, w / 2], [0, 300, h / 2], [0, 0, 1]], np.float64)).astype(np.float32)
+    pose = np.eye(4, dtype=np.float32)
+    pose[:3, 3] = (0.02, -0.01, 0.03)
+    out = [[cuda.full((h, w, 4), 7.0, device="cuda") for _ in range(2)] for _ in range(2)]
+    kf.kernel.raycast(vol, pose, ik, *out[0], min_depth=depths[0], max_depth=depths[1])
+    plain_raycast(kf, cuda, vol, pose, ik, *out[1], (1.99, 0.1), depths)
+    for a, b in zip(*out):
+        assert cuda.equal(a.view(cuda.int32), b.view(cuda.int32))
+    hit = out[1][0][out[1][0][..., 3] == -1]
+    assert (hit[:, 2] < 0).sum() > 1000
