@@ -535,6 +535,7 @@ struct Engine {
     bool has_vis = false;      // some slot has a visualization volume: the step fuses it too
     int slot_fmt = kAnyFormat;   // the volume format every slot has, or kAnyFormat: slots of both
     bool has_range = false;    // some slot's raycast takes depth ranges: the step makes them
+    bool has_trace = false;    // some slot records decision traces (debug)
     unsigned long long* d_ray_counts = nullptr;   // debug mode KF_DEBUG_COUNTERS: raycast work counts
     bool count_rays = false;
     // work-list entries reserved ahead for sessions not open yet (reserve_work)
@@ -766,7 +767,7 @@ struct Engine {
         std::vector<SessionDev> sess(cap);
         std::vector<FuseCtx> fctx(2 * cap, FuseCtx{});
         int max_levels = 1;
-        bool range = false;
+        bool range = false, trace = false;
         int formats = 0;
         for (int s = 0; s < cap; ++s) {
             const Slot& sl = slots[s];
@@ -779,6 +780,7 @@ struct Engine {
             const kf_config& c = sl.cfg;
             max_levels = std::max(max_levels, c.levels);
             range |= sl.d.range != nullptr;
+            trace |= sl.d.trace[0] != nullptr;
             formats |= 1 << sl.d.fmt;
             for (int y = 0; y < c.height; y += kPreTileSize)
                 for (int x = 0; x < c.width; x += kPreTileSize) pre.push_back(PreTile{s, x, y});
@@ -824,6 +826,8 @@ struct Engine {
         slot_fmt = fmt;
         if (range != has_range) graph_dirty = true;   // the step makes depth ranges or not
         has_range = range;
+        if (trace != has_trace) graph_dirty = true;   // the step completes traces or not
+        has_trace = trace;
         KF_TRY(grow(d_pre, cap_pre, std::max<int>(1, int(pre.size()))));
         KF_TRY(grow(d_ray, cap_ray, std::max<int>(1, int(ray.size()))));
         KF_TRY(grow(d_itiles, cap_it, std::max<int>(1, int(all.size()))));
@@ -903,6 +907,7 @@ struct Engine {
         }
         NvtxRange r("kf.raycast");
         if (stages[1]) KF_CK(launch_raycast(v, shape.grid_ray, slot_fmt, st, ray_many));
+        if (stages[1] && has_range && has_trace) KF_CK(launch_count_tails(v, st));
         return KF_OK;
     }
 

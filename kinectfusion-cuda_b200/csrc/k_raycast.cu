@@ -198,7 +198,8 @@ __device__ __forceinline__ void begin_small(RayState& st, float base, float smal
 // rays whose march took the same decisions as another implementation's from rays where a sample
 // near 0.99 or 0 decided differently:
 //   bits 40..  samples taken when the march left large steps (0: it never did)
-//   bits  8..39 samples taken when the march ended (skipped samples count as taken)
+//   bits  8..39 samples taken when the march ended (skipped samples count as taken, and so do those
+//               left to the far plane where a depth range ended the ray: count_tails_kernel)
 //   bits  4..5  how it left large steps: 1 a sample in [0, 0.99), 2 a negative one (back-off)
 //   bits  0..1  how it ended: 0 past the far plane or the sample bound, 1 negative first
 //               sample, 2 refined hit
@@ -224,10 +225,12 @@ enum RayCount {
 };
 
 template <bool kOn> struct MarchCount {
+    static constexpr bool on = false;
     __device__ __forceinline__ void add(int, unsigned int) {}
     __device__ __forceinline__ void flush(unsigned long long*) {}
 };
 template <> struct MarchCount<true> {
+    static constexpr bool on = true;
     unsigned int c[kRayCounts] = {};
     __device__ __forceinline__ void add(int k, unsigned int x) { c[k] += x; }
     __device__ __forceinline__ void flush(unsigned long long* dst) {
@@ -732,10 +735,24 @@ __device__ __forceinline__ void write_trace(const SessionDev* S, int level, int 
     if (tr) tr[size_t(j) * S->lv[level].w + i] = code;
 }
 
+// the work counts' share of the samples between the end of a ray's depth range and its far plane
+template <class Cnt>
+__device__ __forceinline__ void count_tail(const SessionDev* S, const RayGeo& g, float precise, RayState st, Cnt& cnt) {
+    if constexpr (Cnt::on) {
+        RayState whole;
+        if (!S->range || precise != 0.0f || st.t < st.far_d || !ray_start(S, g, whole)) return;
+        if (!(st.t < whole.far_d) || st.guard >= kMaxMarchSamples) return;
+        const int g0 = st.guard;
+        skip_to(st, whole.far_d, S->mu * (st.small ? S->step_s : S->step_l));
+        cnt.add(kCntSkipped, unsigned(st.guard - g0));
+    }
+}
+
 template <class TF, class Cnt>
 __device__ void finish_ray(const SessionDev* S, const RayGeo& g, const TF* f, int level, int i, int j, float precise,
                            const RayState& st, Cnt& cnt) {
     write_trace(S, level, i, j, ray_trace_code(st, precise));
+    count_tail(S, g, precise, st, cnt);
     const HitGeo h = hit_geo(S, g, precise);
     float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (precise != 0.0f) {
@@ -750,7 +767,10 @@ __device__ void finish_ray(const SessionDev* S, const RayGeo& g, const TF* f, in
 template <class TF, class Cnt>
 __device__ void finish_ray_warp(const SessionDev* S, const RayGeo& g, const TF* f, int level, int i, int j,
                                 float precise, int lane, const RayState& st, Cnt& cnt) {
-    if (lane == 0) write_trace(S, level, i, j, ray_trace_code(st, precise));
+    if (lane == 0) {
+        write_trace(S, level, i, j, ray_trace_code(st, precise));
+        count_tail(S, g, precise, st, cnt);
+    }
     const HitGeo h = hit_geo(S, g, precise);
     float mine = 0.f;
     if (precise != 0.0f && lane < 6) {
@@ -927,6 +947,43 @@ __device__ void coop_ray(const SessionDev* S, const LongRay& L, int lane, Cnt& c
     finish_ray_warp(S, g, f, L.level, L.i, L.j, precise, lane, st, cnt);
 }
 
+// The samples that a depth range left out at the end of a ray without a hit: it tells of the decisions in
+// the ray's trace how many the march takes to the far plane.
+__device__ __forceinline__ unsigned long long whole_trace(const SessionDev* S, RayState st, unsigned long long code) {
+    const float large = S->mu * S->step_l;
+    const int sw = int(code >> 40);
+    if (sw) {   // small steps since sample sw - 1 of the large ones
+        const float t = march_pos(st.base, sw - 1, large);
+        st.base = (code >> 4 & 3) == 2 ? __fsub_rn(t, S->mu) : t;
+        st.guard = sw - 1;
+    }
+    skip_to(st, st.far_d, sw ? S->mu * S->step_s : large);
+    return (code & ~(0xffffffffull << 8)) | static_cast<unsigned long long>(st.guard) << 8;
+}
+
+// Debug mode, after the raycast: the traces of rays without a hit as if no depth range had ended them, so
+// that they count what the march counts and 0 means a ray that never marched.
+__global__ void __launch_bounds__(256) count_tails_kernel(EngineView v) {
+    const int lane = threadIdx.x & 31, tw = v.tb->ray_tw;
+    for (int t = blockIdx.x * 8 + (threadIdx.x >> 5); t < v.tb->n_ray; t += gridDim.x * 8) {
+        const RayTile T = v.ray[t];
+        const StepDev st = v.step[T.s];
+        const SessionDev* S = &v.sess[T.s];
+        const LevelDev& Lv = S->lv[T.level];
+        const int i = T.x0 + lane % tw, j = T.y0 + lane / tw;
+        if (!st.active || st.first || !S->range || !S->trace[T.level] || i >= Lv.cw || j >= Lv.ch) continue;
+        unsigned long long* code = S->trace[T.level] + size_t(j) * Lv.w + i;
+        if (*code & 3) continue;
+        float m[9];
+        F3 o;
+        ray_matrix(S, Lv, m, o);
+        RayGeo g;
+        make_geo(S, m, o, i, j, g);
+        RayState ray;
+        if (ray_start(S, g, ray)) *code = whole_trace(S, ray, *code);
+    }
+}
+
 // the queued long rays, one warp each
 template <bool kCount>
 __global__ void __launch_bounds__(256) raycast_long_kernel(EngineView v) {
@@ -981,6 +1038,11 @@ cudaError_t launch_raycast(const EngineView& v, int grid, int fmt, cudaStream_t 
 }
 
 int ray_count_slots() { return kRayCounts; }
+
+cudaError_t launch_count_tails(const EngineView& v, cudaStream_t st) {
+    count_tails_kernel<<<148 * 4, 256, 0, st>>>(v);
+    return cudaGetLastError();
+}
 
 // ---- stage: kernel::raycast on a caller volume, and kf_render on a session's ----
 //

@@ -111,6 +111,8 @@ cudaError_t launch_preprocess(const EngineView& v, int grid, cudaStream_t st);
 // clears the wait record and the counters.
 cudaError_t launch_ray_range(const EngineView& v, int grid, cudaStream_t st);
 cudaError_t launch_raycast(const EngineView& v, int grid, int fmt, cudaStream_t st, bool many);
+// debug mode: the traces of rays without a hit count the samples that depth ranges left out
+cudaError_t launch_count_tails(const EngineView& v, cudaStream_t st);
 int serial_budget_many();   // the lane budget of the raycast's many-tile form
 int ray_count_slots();      // entries of the raycast's debug work counts
 // single: an engine of one slot (the kernel keeps that session's state per block)

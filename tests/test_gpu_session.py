@@ -341,3 +341,37 @@ def test_submitted_frames_equal_synchronous_frames(kf, cuda, run_small):
     assert s2.frame_stats()["frame"] == len(imgs) - 1
     st, pose = s2.process_frame(host[0])   # the queue is empty again
     s2.close()
+
+
+def test_traces_count_the_samples_of_missed_rays(kf, orc, cuda):
+    """A ray without a hit counts its samples to the far plane in its trace, though its tile's depth range
+    lets it stop before: the FP64 oracle's counts for the same volume and pose, but for a sample a
+    rounding away from the far plane (at most 0.1 % of the rays, by one), and 0 only for the rays that
+    never march."""
+    from kfb200 import synth
+    cfg = kf.config_small(volume_n=192, mu=0.03, keep_on_miss=0)
+    imgs, _ = synth.sequence(cfg, 3, seed=5, kind=synth.LOOP)
+    s = kf.KinectFusion(cfg)
+    s.set_debug(kf.KF_DEBUG_RAY_TRACE)
+    for img in imgs[:2]:
+        s.process_frame(img)
+    tracked = s.pose()
+    across = tracked.copy()
+    across[:3, 3] = (0.1, 0.1, 0.0)
+    across[:3, :3] = np.array([[0, 0, 1], [0, 1, 0], [-1, 0, 0]], np.float32)
+    for pose in (tracked, across):
+        f, _ = s.tsdf()
+        s.set_pose(pose)
+        s.process_frame(imgs[2])
+        for level in range(cfg.levels):
+            want = orc.raycast(f, cfg.volume_width, cfg.mu, pose, kf.level_inverse_intrinsics(cfg, level),
+                               cfg.width >> level, cfg.height >> level, cfg.min_depth, cfg.max_depth, cfg.step_large,
+                               cfg.step_small, keep_on_miss=False, prec=1, trace=True, exact_positions=True)[3]
+            got = s.ray_trace(level).astype(np.int64)
+            np.testing.assert_array_equal(got == 0, want == 0)
+            head = np.int64(~((1 << 40) - 1)) | np.int64(0xff)
+            missed = (want != 0) & ((want & 3) == 0) & ((got & head) == (want & head))
+            off = np.abs(((got >> 8) & 0xffffffff) - ((want >> 8) & 0xffffffff))[missed]
+            assert off.size > 50
+            assert off.max() <= 1 and np.mean(off != 0) <= 1e-3, (level, off.max(), float(np.mean(off != 0)))
+    s.close()
