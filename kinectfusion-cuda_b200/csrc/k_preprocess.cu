@@ -21,6 +21,18 @@ namespace kf {
 
 // ---- per-pixel cores shared by the fused kernel and the stage kernels ----
 
+// A tap's weight exp(-s / sigma_s^2 - r / sigma_r^2), s its squared pixel distance and r its squared
+// depth difference: one of the two products is fused into the sum and the other rounded.  Which one is
+// spelled out, because the unrolled and the looped filter are compiled differently and a filtered
+// depth must not depend on that.  kShared rounds the product of the distance, which taps at one
+// distance share: the frame's filter at radii 2 and 3 (the stage's filter rounds the other).  With the
+// reference's sigma_s of 4 that product is exact and the two agree.
+template <bool kShared>
+__device__ __forceinline__ float bilateral_weight(float s, float r, float inv_ss, float inv_sr) {
+    return kShared ? __expf(__fmaf_rn(-r, inv_sr, -__fmul_rn(s, inv_ss)))
+                   : __expf(__fmaf_rn(-s, inv_ss, -__fmul_rn(r, inv_sr)));
+}
+
 // applyBilateralFilterKernel body (project/src/measurement.cu:45-65): x outer, y inner,
 // exp(-dx2/ss^2 - dr2/sr^2) with the fast exponential the reference's fast-math build
 // selects, then acc / norm.  rd(x, y) returns the clamped neighbour.
@@ -34,7 +46,7 @@ __device__ __forceinline__ float bilateral_core(Reader rd, int R, float inv_ss, 
             const float s = float(x * x + y * y);
             float r = center - cur;
             r *= r;
-            const float e = __expf(-s * inv_ss - r * inv_sr);
+            const float e = bilateral_weight<false>(s, r, inv_ss, inv_sr);
             norm += e;
             acc += e * cur;
         }
@@ -43,9 +55,8 @@ __device__ __forceinline__ float bilateral_core(Reader rd, int R, float inv_ss, 
 }
 
 // The same for a radius known at compile time (the configurations' 2 and the reference's 3):
-// the taps unroll with constant offsets into the tile; the arithmetic is the loop's above,
-// operation for operation.
-template <int kR, class Reader>
+// the taps unroll with constant offsets into the tile, in the order of the loop above.
+template <int kR, bool kShared, class Reader>
 __device__ __forceinline__ float bilateral_fixed(Reader rd, float inv_ss, float inv_sr) {
     const float center = rd(0, 0);
     float norm = 0.f, acc = 0.f;
@@ -57,7 +68,7 @@ __device__ __forceinline__ float bilateral_fixed(Reader rd, float inv_ss, float 
             const float s = float(x * x + y * y);
             float r = center - cur;
             r *= r;
-            const float e = __expf(-s * inv_ss - r * inv_sr);
+            const float e = bilateral_weight<kShared>(s, r, inv_ss, inv_sr);
             norm += e;
             acc += e * cur;
         }
@@ -135,8 +146,8 @@ __device__ __forceinline__ void preprocess_tile(const EngineView& v, const PreTi
             if (gx < L0.cw && gy < L0.ch) {
                 const float* c = reg + (ly + R) * pitch + (lx + R);
                 if constexpr (kR > 0)
-                    d = bilateral_fixed<kR>([c](int x, int y) { return c[y * (kPreTileSize + 2 * kR) + x]; },
-                                            S->bil_inv_ss, S->bil_inv_sr);
+                    d = bilateral_fixed<kR, true>([c](int x, int y) { return c[y * (kPreTileSize + 2 * kR) + x]; },
+                                                  S->bil_inv_ss, S->bil_inv_sr);
                 else
                     d = bilateral_core([c, pitch](int x, int y) { return c[y * pitch + x]; }, R, S->bil_inv_ss,
                                        S->bil_inv_sr);
@@ -236,7 +247,7 @@ __global__ void __launch_bounds__(kBilW * kBilH) bilateral_kernel(const float* i
     const float* c = reg + (ly + R) * pitch + lx + R;
     float d;
     if constexpr (kR > 0)
-        d = bilateral_fixed<kR>([c](int x, int y) { return c[y * (kBilW + 2 * kR) + x]; }, inv_ss, inv_sr);
+        d = bilateral_fixed<kR, false>([c](int x, int y) { return c[y * (kBilW + 2 * kR) + x]; }, inv_ss, inv_sr);
     else
         d = bilateral_core([c, pitch](int x, int y) { return c[y * pitch + x]; }, R, inv_ss, inv_sr);
     out[size_t(j) * w + i] = d;

@@ -366,3 +366,25 @@ def test_raycast_behind_the_camera(kf, cuda, n, w, h, fmt, depths):
         assert cuda.equal(a.view(cuda.int32), b.view(cuda.int32))
     hit = out[1][0][out[1][0][..., 3] == -1]
     assert (hit[:, 2] < 0).sum() > 1000
+
+
+@pytest.mark.parametrize("radius", [2, 3])
+@pytest.mark.parametrize("sigma_s,sigma_r", [(4.5, 0.03), (4.0, 0.25), (3.3, 0.11)])
+def test_bilateral_radii_agree(kf, cuda, radius, sigma_s, sigma_r):
+    """A filtered depth does not depend on how the filter is built for its radius: patches as wide as the
+    window, each ringed by depths so far off that their weights are zero, give their middles the same
+    bits at every radius -- the ring adds zeros, in the same order."""
+    cells, side = 40, 9
+    rng = np.random.default_rng(radius)
+    d = np.full((cells * side, cells * side), 900.0, np.float32)
+    inner = slice(4 - radius, 5 + radius)
+    for i in range(cells):
+        for j in range(cells):
+            patch = rng.uniform(0.5, 6.0) + sigma_r * rng.standard_normal((2 * radius + 1, 2 * radius + 1))
+            d[i * side:(i + 1) * side, j * side:(j + 1) * side][inner, inner] = patch
+    mid = []
+    for r in (radius, 4):
+        out = cuda.zeros(d.shape, device="cuda")
+        kf.kernel.applyBilateralFilter(dev(cuda, d), out, sigma_s, sigma_r, r)
+        mid.append(out.cpu().numpy()[4::side, 4::side])
+    np.testing.assert_array_equal(mid[0].view(np.int32), mid[1].view(np.int32))
