@@ -17,6 +17,11 @@
  *     with KF_WEIGHT_SCALE fixed-point steps per unit of weight.  kf_get_tsdf /
  *     kf_set_tsdf convert to and from the reference's interleaved float2 .bin layout
  *     (project/src/voxel_grid.cpp:43-80).
+ *   - Device arrays that the kernels access as vectors start on one, else the call is refused with
+ *     KF_ERR_ARG: vertex and normal maps on 16 bytes; a kf_volume's arrays on 16 bytes for
+ *     kf_initialize_grid and, for kf_fuse, on four voxels (16 bytes, or 8 in KF_TSDF_F16U16; kf_raycast
+ *     takes any voxel); RGBA images on 4 bytes; the interleaved TSDF of kf_get_tsdf / kf_set_tsdf in
+ *     device memory on 8.
  *   - Every call returns a kf_status; nothing throws across this boundary.  Where the
  *     reference throws std::runtime_error on a shape mismatch (e.g.
  *     project/src/measurement.cu:144-147) this ABI returns KF_ERR_SHAPE.

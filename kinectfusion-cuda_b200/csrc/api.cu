@@ -52,6 +52,13 @@ thread_local cudaError_t g_last_cuda = cudaSuccess;
 
 inline cudaStream_t as_stream(void* s) { return static_cast<cudaStream_t>(s); }
 
+// The kernels read and write some arrays as wider vectors than their C type says (kf_api.h); a pointer
+// that does not start on one would fault on the device, so it is refused here.
+template <class... P>
+bool aligned(size_t to, const P*... p) {
+    return ((reinterpret_cast<uintptr_t>(p) % to == 0) && ...);
+}
+
 // ---- configuration ----
 
 kf_status validate(const kf_config& c) {
@@ -1524,6 +1531,7 @@ static kf_status copy_grid_out(const void* tf, const void* tw, int n, int fmt, v
     }
     if (layout != 1) return KF_ERR_ARG;
     if (dst_bytes < n3 * 8) return KF_ERR_SHAPE;
+    if (!to_host && !aligned(8, dst)) return KF_ERR_ARG;
     float* tmp = nullptr;
     if (to_host) KF_CK(cudaMalloc(&tmp, n3 * 8));
     float* target = to_host ? tmp : static_cast<float*>(dst);
@@ -1563,6 +1571,7 @@ static kf_status copy_grid_in(void* tf, void* tw, int n, int fmt, int* bmin, int
     } else {
         if (layout != 1) return KF_ERR_ARG;
         if (src_bytes < n3 * 8) return KF_ERR_SHAPE;
+        if (!from_host && !aligned(8, src)) return KF_ERR_ARG;
         float* tmp = nullptr;
         const float* from = static_cast<const float*>(src);
         if (from_host) {
@@ -1687,7 +1696,8 @@ kf_status kf_session_checkpoint_load(kf_session* s, const char* path) {
 
 static kf_status display(int mode, const void* src, int w, int h, const DispMats& m, float scale, uint8_t* rgba,
                          void* stream, float* elapsed_ms) {
-    if (!src || !rgba || w <= 0 || h <= 0) return KF_ERR_ARG;
+    if (!src || !rgba || w <= 0 || h <= 0 || !aligned(mode == kDisplayFloat ? 4 : 16, src) || !aligned(4, rgba))
+        return KF_ERR_ARG;
     StageTimer t(elapsed_ms, as_stream(stream));
     return t.finish(stage_display(mode, src, w, h, m, scale, reinterpret_cast<unsigned int*>(rgba), as_stream(stream)));
 }
@@ -1831,7 +1841,7 @@ kf_status kf_down_sample(const float* in, int w, int h, float* out, int out_w, i
 
 kf_status kf_create_vertex_map(const float* depth, int w, int h, float* vertex, int out_w, int out_h,
                                const float inv_cam_k[9], void* stream, float* elapsed_ms) {
-    if (!depth || !vertex || !inv_cam_k || w <= 0 || h <= 0) return KF_ERR_ARG;
+    if (!depth || !vertex || !inv_cam_k || w <= 0 || h <= 0 || !aligned(16, vertex)) return KF_ERR_ARG;
     if (w != out_w || h != out_h) return KF_ERR_SHAPE;
     StageTimer t(elapsed_ms, as_stream(stream));
     return t.finish(stage_vertex(depth, reinterpret_cast<float4*>(vertex), w, h, inv_cam_k, as_stream(stream)));
@@ -1839,7 +1849,7 @@ kf_status kf_create_vertex_map(const float* depth, int w, int h, float* vertex, 
 
 kf_status kf_create_normal_map(const float* vertex, int w, int h, float* normal, int out_w, int out_h, void* stream,
                                float* elapsed_ms) {
-    if (!vertex || !normal || w <= 0 || h <= 0) return KF_ERR_ARG;
+    if (!vertex || !normal || w <= 0 || h <= 0 || !aligned(16, vertex, normal)) return KF_ERR_ARG;
     if (w != out_w || h != out_h) return KF_ERR_SHAPE;
     StageTimer t(elapsed_ms, as_stream(stream));
     return t.finish(stage_normal(reinterpret_cast<const float4*>(vertex), reinterpret_cast<float4*>(normal), w, h,
@@ -1855,6 +1865,7 @@ static kf_status check_volume(const kf_volume* v) {
 
 kf_status kf_initialize_grid(const kf_volume* vol, void* stream, float* elapsed_ms) {
     KF_TRY(check_volume(vol));
+    if (!aligned(16, vol->f, vol->w)) return KF_ERR_ARG;
     const long long n3 = (long long)vol->n * vol->n * vol->n;
     StageTimer t(elapsed_ms, as_stream(stream));
     return t.finish(launch_init_volume(vol->f, vol->w, n3, vol->format, as_stream(stream)));
@@ -1865,6 +1876,7 @@ kf_status kf_fuse(const float* depth_m, int w, int h, const float cam_k[9], cons
     NvtxRange nvtx_("kf_fuse");
     if (!depth_m || !cam_k || !pose || w <= 0 || h <= 0) return KF_ERR_ARG;
     KF_TRY(check_volume(vol));
+    if (!aligned(vol->format == KF_TSDF_F16U16 ? 8 : 16, vol->f, vol->w)) return KF_ERR_ARG;   // four voxels
     cudaStream_t st = as_stream(stream);
     Scratch scratch;
     KF_CK(scratch.take(stage_fuse_scratch(vol->n, w, h), st));
@@ -1880,6 +1892,7 @@ kf_status kf_raycast(const kf_volume* vol, const float pose[16], const float inv
     NvtxRange nvtx_("kf_raycast");
     if (!pose || !inv_cam_k || !vertex || !normal || w <= 0 || h <= 0) return KF_ERR_ARG;
     KF_TRY(check_volume(vol));
+    if (!aligned(16, vertex, normal) || !aligned(vol->format == KF_TSDF_F16U16 ? 2 : 4, vol->f)) return KF_ERR_ARG;
     if (w != nw || h != nh) return KF_ERR_SHAPE;   // project/src/raycast.cu:155-158
     if (!(step_large > step_small) || !(max_depth > min_depth) || !(max_depth < 1000.f) ||
         !(vol->mu * step_small > max_depth * 1e-6f))
@@ -1900,7 +1913,7 @@ kf_status kf_construct_icp_residuals(const float* vertex, const float* target_ve
                                      const float cur_transl[3], const float cam_k[9], float distance_thresh,
                                      float angle_thresh, float* mat_a, float* vec_b, void* stream, float* elapsed_ms) {
     if (!vertex || !target_vertex || !target_normal || !prev_rot || !prev_transl || !cur_rot || !cur_transl ||
-        !cam_k || !mat_a || !vec_b || w <= 0 || h <= 0)
+        !cam_k || !mat_a || !vec_b || w <= 0 || h <= 0 || !aligned(16, vertex, target_vertex, target_normal))
         return KF_ERR_ARG;
     StageTimer t(elapsed_ms, as_stream(stream));
     return t.finish(stage_icp_residuals(reinterpret_cast<const float4*>(vertex),
@@ -1968,7 +1981,9 @@ kf_status kf_compute_pose(const float* const* vertex, const float* const* target
     for (int l = 0; l < levels; ++l) total += std::max(0, c.iters[l]);
     if (total > kIcpMaxPasses) return KF_ERR_ARG;
     for (int l = 0; l < levels; ++l)
-        if (!vertex[l] || !target_vertex[l] || !target_normal[l]) return KF_ERR_ARG;
+        if (!vertex[l] || !target_vertex[l] || !target_normal[l] ||
+            !aligned(16, vertex[l], target_vertex[l], target_normal[l]))
+            return KF_ERR_ARG;
     cudaStream_t s = as_stream(stream);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     KF_CK(cudaStreamIsCapturing(s, &cs));

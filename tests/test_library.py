@@ -138,3 +138,51 @@ def test_level_inverse_intrinsics(kf, level):
         ik = kf.level_inverse_intrinsics(cfg, level)
         assert ik.dtype == np.float32
         np.testing.assert_allclose(ik.astype(np.float64) @ k, np.eye(3), atol=2e-6)
+
+
+@pytest.mark.parametrize("fmt,need_f,need_w", [(0, 16, 16), (1, 8, 8)])
+def test_volumes_and_maps_off_their_alignment_are_refused(kf, fmt, need_f, need_w):
+    """The stage calls read and write volumes, float4 maps and RGBA images as vectors; pointers that do not
+    start on one are refused on the host, before any device work.  No address here is ever read."""
+    at = 0x10000000
+    m9, m16 = kf.to_colmajor(np.eye(3, dtype=np.float32)), kf.to_colmajor(np.eye(4, dtype=np.float32))
+    t3 = (ctypes.c_float * 3)()
+
+    def vol(df, dw):
+        return ctypes.byref(kf._lib.KfVolume(at + df, at + dw, 64, 2.0, 0.1, fmt, 0.0))
+
+    def ptr(d=0):
+        return ctypes.c_void_p(at + d)
+
+    def maps(d):
+        return (ctypes.c_void_p * 3)(at, at + d, at)
+
+    L, A = kf.lib, kf.KF_ERR_ARG
+    es = 2 if fmt else 4
+    for d in (1, es, need_f // 2, need_f + es):
+        assert L.kf_fuse(ptr(), 32, 24, m9, vol(d, 0), m16, 0.4, 6.0, None, None) == A
+        assert L.kf_fuse(ptr(), 32, 24, m9, vol(0, d), m16, 0.4, 6.0, None, None) == A
+    for d in (1, es, 8, 16 + es):
+        assert L.kf_initialize_grid(vol(d, 0), None, None) == A
+        assert L.kf_initialize_grid(vol(0, d), None, None) == A
+    for d in range(1, es):
+        assert L.kf_raycast(vol(d, 0), m16, m9, ptr(), 32, 24, ptr(), 32, 24, 0.4, 6.0, 1.99, 0.1, None, None) == A
+    cfg = kf.config_small()
+    for d in (1, 4, 8, 20):
+        v = vol(0, 0)
+        assert L.kf_raycast(v, m16, m9, ptr(d), 32, 24, ptr(), 32, 24, 0.4, 6.0, 1.99, 0.1, None, None) == A
+        assert L.kf_raycast(v, m16, m9, ptr(), 32, 24, ptr(d), 32, 24, 0.4, 6.0, 1.99, 0.1, None, None) == A
+        assert L.kf_create_vertex_map(ptr(), 32, 24, ptr(d), 32, 24, m9, None, None) == A
+        assert L.kf_create_normal_map(ptr(d), 32, 24, ptr(), 32, 24, None, None) == A
+        assert L.kf_create_normal_map(ptr(), 32, 24, ptr(d), 32, 24, None, None) == A
+        for k in range(3):
+            p = [ptr(d if q == k else 0) for q in range(3)]
+            assert L.kf_construct_icp_residuals(*p, 32, 24, m9, t3, m9, t3, m9, 0.1, 0.3, ptr(), ptr(), None, None) == A
+            p = [maps(d if q == k else 0) for q in range(3)]
+            assert L.kf_compute_pose(*p, 32, 24, 3, ctypes.byref(cfg), m16, m16, None, None) == A
+        assert L.kf_normal_map_to_rgba(ptr(d), 32, 24, m9, ptr(), None, None) == A
+        assert L.kf_shading_to_rgba(ptr(d), 32, 24, m16, m9, ptr(), None, None) == A
+    for d in (1, 2, 3):
+        assert L.kf_normal_map_to_rgba(ptr(), 32, 24, m9, ptr(d), None, None) == A
+        assert L.kf_shading_to_rgba(ptr(), 32, 24, m16, m9, ptr(d), None, None) == A
+        assert L.kf_float_channel_to_rgba(ptr(), 32, 24, 1.0, ptr(d), None, None) == A
