@@ -221,7 +221,8 @@ kf_status kf_create_normal_map(const float* vertex, int w, int h, float* normal,
 /* kernel::initializeGrid, project/src/tsdf.cuh:15 (value {f = 2, w = 0}) */
 kf_status kf_initialize_grid(const kf_volume* vol, void* stream, float* elapsed_ms);
 /* kernel::fuse, project/src/tsdf.cuh:16.  cam_k: level-0 intrinsics, column-major;
- * w, h: the frustum bounds (the reference hard-codes 640 x 480). */
+ * w, h: the frustum bounds (the reference hard-codes 640 x 480).  Synchronizes `stream`; a stream
+ * that is being captured is refused (KF_ERR_CUDA) before anything is recorded. */
 kf_status kf_fuse(const float* depth_m, int w, int h, const float cam_k[9], const kf_volume* vol,
                   const float pose[16], float min_depth, float max_depth, void* stream,
                   float* elapsed_ms);

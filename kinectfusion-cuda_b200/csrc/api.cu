@@ -1148,6 +1148,16 @@ void raycast_scratch(Scratch& scratch, int n, int w, int h, int longq_cap, cudaS
         cudaGetLastError();
 }
 
+// A call that waits for its stream cannot be captured: an error before anything is recorded, so that the
+// caller's capture goes on.
+kf_status refuse_capture(cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    KF_CK(cudaStreamIsCapturing(st, &cs));
+    if (cs == cudaStreamCaptureStatusNone) return KF_OK;
+    g_last_cuda = cudaErrorStreamCaptureUnsupported;
+    return KF_ERR_CUDA;
+}
+
 // event pair around a stage call when the caller asks for its time (the reference's
 // kernel:: wrappers all return elapsed milliseconds)
 struct StageTimer {
@@ -1878,12 +1888,15 @@ kf_status kf_fuse(const float* depth_m, int w, int h, const float cam_k[9], cons
     KF_TRY(check_volume(vol));
     if (!aligned(vol->format == KF_TSDF_F16U16 ? 8 : 16, vol->f, vol->w)) return KF_ERR_ARG;   // four voxels
     cudaStream_t st = as_stream(stream);
+    KF_TRY(refuse_capture(st));
     Scratch scratch;
     KF_CK(scratch.take(stage_fuse_scratch(vol->n, w, h), st));
     StageTimer t(elapsed_ms, st);
-    kf_status r = t.finish(stage_fuse(depth_m, w, h, cam_k, vol, pose, min_depth, max_depth, scratch.p, st));
-    cudaStreamSynchronize(st);
-    return r;
+    const kf_status r = t.finish(stage_fuse(depth_m, w, h, cam_k, vol, pose, min_depth, max_depth, scratch.p, st));
+    const cudaError_t e = cudaStreamSynchronize(st);
+    KF_TRY(r);
+    KF_CK(e);
+    return KF_OK;
 }
 
 kf_status kf_raycast(const kf_volume* vol, const float pose[16], const float inv_cam_k[9], float* vertex, int w, int h,
@@ -1985,12 +1998,7 @@ kf_status kf_compute_pose(const float* const* vertex, const float* const* target
             !aligned(16, vertex[l], target_vertex[l], target_normal[l]))
             return KF_ERR_ARG;
     cudaStream_t s = as_stream(stream);
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    KF_CK(cudaStreamIsCapturing(s, &cs));
-    if (cs != cudaStreamCaptureStatusNone) {   // the pose comes back to the host: not capturable
-        g_last_cuda = cudaErrorStreamCaptureUnsupported;
-        return KF_ERR_CUDA;
-    }
+    KF_TRY(refuse_capture(s));   // the pose comes back to the host
     // maps written on the default stream may be passed with any stream
     if (s) KF_CK(cudaStreamSynchronize(nullptr));
 

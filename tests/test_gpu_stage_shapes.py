@@ -388,3 +388,31 @@ def test_bilateral_radii_agree(kf, cuda, radius, sigma_s, sigma_r):
         kf.kernel.applyBilateralFilter(dev(cuda, d), out, sigma_s, sigma_r, r)
         mid.append(out.cpu().numpy()[4::side, 4::side])
     np.testing.assert_array_equal(mid[0].view(np.int32), mid[1].view(np.int32))
+
+
+def test_fuse_refuses_a_captured_stream(kf, cuda):
+    """kf_fuse waits for its stream, so a stream that is being captured is refused with an error, before
+    anything is recorded: the capture goes on and the volume is untouched."""
+    import ctypes
+    n, w, h = 64, 64, 48
+    f, wt = cuda.full((n, n, n), 2.0, device="cuda"), cuda.zeros((n, n, n), device="cuda")
+    vol = kf.kernel.volume(f, wt, 2.0, 0.1)
+    depth, other = cuda.full((h, w), 1.0, device="cuda"), cuda.zeros(1, device="cuda")
+    k = np.array([[60, 0, w / 2], [0, 60, h / 2], [0, 0, 1]], np.float32)
+    pose = np.eye(4, dtype=np.float32)
+    pose[2, 3] = -1.0
+    s = cuda.cuda.Stream()
+    ms = ctypes.c_float()
+    cuda.cuda.synchronize()
+    g, got = cuda.cuda.CUDAGraph(), []
+    with cuda.cuda.graph(g, stream=s):
+        for elapsed in (None, ctypes.byref(ms)):
+            got.append(kf.lib.kf_fuse(ctypes.c_void_p(depth.data_ptr()), w, h, kf.to_colmajor(k), ctypes.byref(vol),
+                                      kf.to_colmajor(pose), 0.4, 6.0, ctypes.c_void_p(s.cuda_stream), elapsed))
+        other.add_(1)
+    assert got == [kf.KF_ERR_CUDA] * 2
+    g.replay()
+    cuda.cuda.synchronize()
+    assert float(other) == 1 and float(wt.max()) == 0
+    kf.kernel.fuse(depth, vol, pose, k)
+    assert float(wt.max()) > 0
