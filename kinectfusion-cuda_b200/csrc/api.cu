@@ -884,14 +884,12 @@ struct Engine {
             KF_CK(cudaEventRecord(ev_fork, st));
             KF_CK(cudaStreamWaitEvent(aux_stream, ev_fork, 0));
             if (input_wait) KF_CK(cudaStreamWaitEvent(aux_stream, ev_input, capturing ? cudaEventWaitExternal : 0));
-            NvtxRange r("kf.preprocess");
-            KF_CK(launch_preprocess(v, shape.grid_pre, aux_stream));
+            KF_TRY(record_preprocess(v, aux_stream));
             if (profile) KF_CK(cudaEventRecordWithFlags(ev[1], aux_stream, cudaEventRecordExternal));
             KF_CK(cudaEventRecord(ev_join, aux_stream));
         } else {
             if (stages[0] && input_wait) KF_CK(cudaStreamWaitEvent(st, ev_input, capturing ? cudaEventWaitExternal : 0));
-            NvtxRange r("kf.preprocess");
-            if (stages[0]) KF_CK(launch_preprocess(v, shape.grid_pre, st));
+            if (stages[0]) KF_TRY(record_preprocess(v, st));
             if (profile) KF_CK(cudaEventRecordWithFlags(ev[1], st, cudaEventRecordExternal));
         }
         KF_TRY(record_raycast(v, st));
@@ -904,7 +902,14 @@ struct Engine {
         return KF_OK;
     }
 
+    kf_status record_preprocess(const EngineView& v, cudaStream_t st) {
+        NvtxRange r("kf.preprocess");
+        KF_CK(launch_preprocess(v, shape.grid_pre, st));
+        return KF_OK;
+    }
+
     kf_status record_raycast(const EngineView& v, cudaStream_t st) {
+        NvtxRange r("kf.raycast");
         // clear the wait record and the counters; the depth-range launch does it on the way
         if (has_range) {
             const int units_grid = int(std::min<long long>((tb.fuse_total + 255) / 256, sms * 4));
@@ -912,7 +917,6 @@ struct Engine {
         } else {
             KF_CK(cudaMemsetAsync(d_sync, 0, sizeof(GridSync) + sizeof(unsigned int) * kCounters, st));
         }
-        NvtxRange r("kf.raycast");
         if (stages[1]) KF_CK(launch_raycast(v, shape.grid_ray, slot_fmt, st, ray_many));
         if (stages[1] && has_range && has_trace) KF_CK(launch_count_tails(v, st));
         return KF_OK;
@@ -1006,7 +1010,7 @@ struct Engine {
         const EngineView v = view();
         KF_TRY(record_raycast(v, st));
         KF_TRY(copy(cs));
-        KF_CK(launch_preprocess(v, shape.grid_pre, cs));
+        KF_TRY(record_preprocess(v, cs));
         KF_TRY(end_inputs(cs));
         KF_CK(cudaStreamWaitEvent(st, ev_input, 0));
         KF_TRY(record_pose(v, st));

@@ -375,3 +375,49 @@ def test_traces_count_the_samples_of_missed_rays(kf, orc, cuda):
             assert off.size > 50
             assert off.max() <= 1 and np.mean(off != 0) <= 1e-3, (level, off.max(), float(np.mean(off != 0)))
     s.close()
+
+
+NVTX_LOG = r"""
+#include <stddef.h>
+#include <string.h>
+#include <unistd.h>
+/* an NVTX tool that writes the name of every range pushed to descriptor 2 */
+typedef void (*fn)(void);
+struct callbacks { size_t size; int (*table)(int module, fn*** out, unsigned int* size); };
+static int push(const char* name) { write(2, "nvtx ", 5); write(2, name, strlen(name)); write(2, "\n", 1); return 0; }
+int InitializeInjectionNvtx2(const void* (*get)(unsigned int)) {
+    const struct callbacks* c = get(1);
+    fn** t = 0;
+    unsigned int n = 0;
+    if (!c || !c->table(1, &t, &n) || n <= 9) return 0;
+    *t[9] = (fn)push;   /* nvtxRangePushA */
+    return 1;
+}
+"""
+
+
+def test_every_stage_has_its_nvtx_range(kf, tmp_path):
+    """KF_DEBUG_NO_GRAPH: the four stages of a frame run inside their ranges, from pageable frames (whose
+    raycast starts before the copy) and from device frames."""
+    import subprocess
+    import sys
+    src, so = tmp_path / "nvtx_log.c", tmp_path / "nvtx_log.so"
+    src.write_text(NVTX_LOG)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-w", "-o", str(so), str(src)], check=True)
+    prog = ("import sys, torch; sys.path[:0] = %r\n"
+            "import kfb200 as kf\nfrom kfb200 import synth\n"
+            "cfg = kf.config_small()\nimgs, _ = synth.sequence(cfg, 2, seed=3)\n"
+            "for on_device in (0, 1):\n"
+            "    s = kf.KinectFusion(cfg)\n    s.set_debug(kf.KF_DEBUG_NO_GRAPH)\n"
+            "    for img in imgs:\n"
+            "        sys.stderr.write('next one\\n'); sys.stderr.flush()\n"
+            "        s.process_frame(torch.from_numpy(img.view('int16')).cuda() if on_device else img)\n"
+            "    s.close()\n" % [os.path.dirname(os.path.dirname(os.path.abspath(kf.__file__)))])
+    r = subprocess.run([sys.executable, "-c", prog], env=dict(os.environ, NVTX_INJECTION64_PATH=str(so)),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    frames = [f.splitlines() for f in r.stderr.split("next one\n")[1:]]
+    assert len(frames) == 4
+    for f in frames:
+        for stage in ("preprocess", "raycast", "icp", "fusion"):
+            assert f.count("nvtx kf." + stage) == 1, f
