@@ -833,15 +833,16 @@ __global__ void __launch_bounds__(256) icp_rows_kernel(const float4* vm, const f
                                                        IcpStageMats m, float dist, float cos_th, float* A, float* b) {
     __shared__ float rows[8][32 * 6];
     const int lane = threadIdx.x, warp = threadIdx.y;
-    const int u = blockIdx.x * 32 + lane, vv = blockIdx.y * 8 + warp;
+    const int u = blockIdx.x * 32 + lane;
+    const unsigned int vv = (blockIdx.z * gridDim.y + blockIdx.y) * 8 + warp;   // h rounded up may pass 2^31
     float a[6], bb;
-    const bool inside = u < w && vv < h;
-    const bool ok = inside && icp_pixel(vm, tv, tn, w, h, u, vv, m.R, m.t, m.M, m.tp, dist, cos_th, a, bb);
+    const bool inside = u < w && vv < unsigned(h);
+    const bool ok = inside && icp_pixel(vm, tv, tn, w, h, u, int(vv), m.R, m.t, m.M, m.tp, dist, cos_th, a, bb);
 #pragma unroll
     for (int q = 0; q < 6; ++q) rows[warp][lane * 6 + q] = ok ? a[q] : 0.f;
     if (inside) b[size_t(vv) * w + u] = ok ? bb : 0.f;
     __syncwarp();
-    if (vv >= h) return;
+    if (vv >= unsigned(h)) return;
     const int floats = 6 * min(32, w - int(blockIdx.x) * 32);
     float* out = A + (size_t(vv) * w + blockIdx.x * 32) * 6;
 #pragma unroll
@@ -862,7 +863,9 @@ cudaError_t stage_icp_residuals(const float4* vmap, const float4* tv, const floa
             for (int q = 0; q < 3; ++q) acc += k[q * 3 + row] * Rp[q * 3 + col];   // K(row,q) * Rp^T(q,col) = K(row,q) * Rp(col,q)
             m.M[col * 3 + row] = acc;
         }
-    dim3 blk(32, 8), grd((w + 31) / 32, (h + 7) / 8);
+    // a grid's second dimension holds 65,535 blocks, 524,280 rows: taller maps go on in the third
+    const unsigned int down = unsigned((h + 7) / 8), most = 65535;
+    const dim3 blk(32, 8), grd((w + 31) / 32, std::min(down, most), (down + most - 1) / most);
     const float cos_th = float(std::cos(double(angle)));
     icp_rows_kernel<<<grd, blk, 0, st>>>(vmap, tv, tn, w, h, m, dist, cos_th, A, b);
     return cudaGetLastError();

@@ -416,3 +416,29 @@ def test_fuse_refuses_a_captured_stream(kf, cuda):
     assert float(other) == 1 and float(wt.max()) == 0
     kf.kernel.fuse(depth, vol, pose, k)
     assert float(wt.max()) > 0
+
+
+@pytest.mark.parametrize("w,h", [(1, 524281), (3, 1048560)])
+def test_icp_rows_of_tall_maps(kf, orc, cuda, w, h):
+    """More rows than a grid's second dimension holds blocks of eight: every row is written, the residual
+    of the one pixel near the bottom that has a normal and zeros for the others."""
+    maps = [cuda.zeros((h, w, 4), device="cuda") for _ in range(3)]
+    for m in maps:
+        m[..., 3] = -2
+    corner = np.array([[[0, 0, 1.01, -1], [0.01, 0, 1.01, -1]], [[0, 0.01, 1.01, -1], [0, 0, 0, -2]]], np.float32)
+    normal = orc.normal_map(corner)[0, 0]
+    if w > 1:
+        maps[0][h - 2:, :2] = dev(cuda, corner)
+        maps[1][h - 2, 0] = cuda.tensor([0.0, 0.0, 1.0, -1.0])
+        maps[2][h - 2, 0] = dev(cuda, normal)
+    k = np.array([[1, 0, 0.5], [0, 1, h - 1.5], [0, 0, 1]], np.float32)
+    eye, zero = np.eye(3, dtype=np.float32), np.zeros(3, np.float32)
+    A, b = cuda.full((w * h, 6), 7.0, device="cuda"), cuda.full((w * h,), 7.0, device="cuda")
+    kf.kernel.constructIcpResiduals(*maps, eye, zero, eye, zero, k, 0.1, 0.35, A, b)
+    if w > 1:
+        at = (h - 2) * w
+        np.testing.assert_allclose(A[at].cpu().numpy(), [0, 0, 0, 0, 0, normal[2]], atol=1e-6)
+        np.testing.assert_allclose(float(b[at]), -0.01 * normal[2], atol=1e-6)
+        A[at] = 0
+        b[at] = 0
+    assert float(A.abs().max()) == 0 and float(b.abs().max()) == 0
