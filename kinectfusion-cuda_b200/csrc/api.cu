@@ -988,18 +988,25 @@ struct Engine {
         return KF_OK;
     }
 
-    // One step with its frames' copies.  copy(cs) puts them on stream cs; `src` is one of the frames
-    // (host memory unless `device`).
+    // One step with its frames' copies.  copy(cs) puts them on stream cs; `src` is one of the `frames`
+    // frames (host memory unless `device`), which have `bytes` in all.
     //
     // A copy from pageable memory holds the calling thread until the frame is staged (some 50 us for
     // 640x480), so the raycast, which needs only earlier frames, is launched before it, and the rest
     // launch by launch while the raycast runs: 640x480 in 512^3 241 -> 219 us a frame, 320x240 in 128^3
-    // 142 -> 137.  Any other copy returns at once, and one graph launch costs less than seven: the whole
+    // 135 -> 131.  Any other copy returns at once, and one graph launch costs less than seven: the whole
     // step is one.  Profiled and counted steps, and steps on a stream that is being captured, too.
+    //
+    // So are steps whose copies take too little of the thread's time: a copy costs it a share for its call
+    // and one for its bytes.  Graph against launches, us: a frame of 64x48 in 256^3 91 / 101, 160x120 in
+    // 128^3 135 / 137, 256x192 130 / 132, 272x204 130 / 130, 320x240 135 / 131; two sessions of 64x48 89 /
+    // 94, of 160x120 184 / 179; three of 64x48 95 / 98, four 100 / 99, twelve 136 / 117.
+    static constexpr size_t kSplitCall = 32 << 10, kSplitBytes = 136 << 10;
+
     template <class Copy>
-    kf_status step(cudaStream_t st, const void* src, bool device, Copy&& copy) {
+    kf_status step(cudaStream_t st, const void* src, bool device, int frames, size_t bytes, Copy&& copy) {
         cudaStream_t cs = st;
-        if (!split_step(st, src, device)) {
+        if (frames * kSplitCall + bytes < kSplitBytes || !split_step(st, src, device)) {
             KF_TRY(begin_inputs(st, &cs));
             KF_TRY(copy(cs));
             KF_TRY(end_inputs(cs));
@@ -1377,7 +1384,7 @@ static kf_status session_enqueue(kf_session* s, const uint16_t* depth, int is_de
     want[s->slot] = StepDev{1, sl.frames == 0 ? 1 : 0};
     KF_TRY(s->eng->set_step(want, st));
     Engine& e = *s->eng;
-    return e.step(st, depth, is_dev != 0, [&](cudaStream_t cs) -> kf_status {
+    return e.step(st, depth, is_dev != 0, 1, bytes, [&](cudaStream_t cs) -> kf_status {
         KF_CK(cudaMemcpyAsync(const_cast<uint16_t*>(sl.d.raw), depth, bytes,
                               is_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, cs));
         return KF_OK;
@@ -2130,8 +2137,15 @@ kf_status kf_batch_step(kf_batch* b, const uint16_t* const* depth, int is_device
     KF_TRY(b->eng.set_step(want, st));
     KF_TRY(tuner_before_step(b->eng));
     const uint16_t* first = nullptr;
-    for (int i = 0; i < b->n && !first; ++i) first = depth[i];
-    KF_TRY(b->eng.step(st, first, is_device_ptr != 0 || !first, [&](cudaStream_t cs) -> kf_status {
+    int frames = 0;
+    size_t bytes = 0;
+    for (int i = 0; i < b->n; ++i) {
+        if (!depth[i]) continue;
+        if (!first) first = depth[i];
+        ++frames;
+        bytes += size_t(b->eng.slots[i].cfg.width) * b->eng.slots[i].cfg.height * 2;
+    }
+    KF_TRY(b->eng.step(st, first, is_device_ptr != 0 || !first, frames, bytes, [&](cudaStream_t cs) -> kf_status {
         for (int i = 0; i < b->n; ++i) {
             if (!depth[i]) continue;
             Slot& sl = b->eng.slots[i];

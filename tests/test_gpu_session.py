@@ -421,3 +421,31 @@ def test_every_stage_has_its_nvtx_range(kf, tmp_path):
     for f in frames:
         for stage in ("preprocess", "raycast", "icp", "fusion"):
             assert f.count("nvtx kf." + stage) == 1, f
+
+
+def test_small_pageable_frames_are_one_graph(kf, tmp_path):
+    """A step whose frames are copied in next to no time is one graph launch, which opens no stage's range;
+    larger frames, or many, have their stages launched around the copies."""
+    import subprocess
+    import sys
+    src, so = tmp_path / "nvtx_log.c", tmp_path / "nvtx_log.so"
+    src.write_text(NVTX_LOG)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-w", "-o", str(so), str(src)], check=True)
+    prog = ("import sys; sys.path[:0] = %r\n"
+            "import kfb200 as kf\nfrom kfb200 import synth\n"
+            "for w, h, n in ((64, 48, 1), (240, 180, 1), (320, 240, 1), (64, 48, 2), (64, 48, 12), (160, 120, 4)):\n"
+            "    cfg = kf.config_small(width=w, height=h, cx=w / 2 - 0.5, cy=h / 2 - 0.5, fx=0.8 * w, fy=0.8 * w, volume_n=64,\n"
+            "                          mu=0.06)\n"
+            "    imgs, _ = synth.sequence(cfg, 4, seed=3)\n"
+            "    s = kf.KinectFusion(cfg) if n == 1 else kf.Batch([cfg] * n)\n"
+            "    for i, img in enumerate(imgs):\n"
+            "        if i == 3:\n"
+            "            sys.stderr.write('next one\\n'); sys.stderr.flush()\n"
+            "        s.process_frame(img) if n == 1 else s.step([img] * n)\n"
+            "    sys.stderr.write('next one\\n'); sys.stderr.flush()\n"
+            "    s.close()\n" % [os.path.dirname(os.path.dirname(os.path.abspath(kf.__file__)))])
+    r = subprocess.run([sys.executable, "-c", prog], env=dict(os.environ, NVTX_INJECTION64_PATH=str(so)),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    last = [f.splitlines() for f in r.stderr.split("next one\n")[1::2]]   # every session's fourth frame
+    assert [f.count("nvtx kf.raycast") for f in last] == [0, 0, 1, 0, 1, 1]
