@@ -1126,10 +1126,21 @@ cudaError_t scratch_pool(cudaMemPool_t* out) {
     return cudaSuccess;
 }
 
+// While another stream is captured, pool calls on this one would break that capture unless the thread
+// says that they have nothing to do with it.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+    RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+};
+
 struct Scratch {
     void* p = nullptr;
     cudaStream_t st = nullptr;
     cudaError_t take(size_t bytes, cudaStream_t s) {
+        RelaxedCapture relaxed;
         cudaMemPool_t pool = nullptr;
         cudaError_t e = scratch_pool(&pool);
         if (e != cudaSuccess) return e;
@@ -1139,7 +1150,11 @@ struct Scratch {
         return e;
     }
     Scratch() = default;
-    ~Scratch() { if (p) cudaFreeAsync(p, st); }
+    ~Scratch() {
+        if (!p) return;
+        RelaxedCapture relaxed;
+        cudaFreeAsync(p, st);
+    }
     Scratch(const Scratch&) = delete;
     Scratch& operator=(const Scratch&) = delete;
 };

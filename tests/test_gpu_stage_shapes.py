@@ -442,3 +442,36 @@ def test_icp_rows_of_tall_maps(kf, orc, cuda, w, h):
         A[at] = 0
         b[at] = 0
     assert float(A.abs().max()) == 0 and float(b.abs().max()) == 0
+
+
+@pytest.mark.parametrize("mode", ["global", "thread_local"])
+def test_raycast_beside_a_capture(kf, orc, cuda, mode):
+    """A raycast on one stream while another is captured: the capture goes on and replays, and the maps are
+    those of a call without one.  In a process of its own, whose first scratch this call takes."""
+    import os
+    import subprocess
+    import sys
+    prog = ("import sys, ctypes; sys.path[:0] = %r\n"
+            "import numpy as np, torch, kfb200 as kf\n"
+            "n, w, h = 64, 480, 360\n"
+            "r = (torch.arange(n, device='cuda') + 0.5) / n * 2 - 1\n"
+            "z, y, x = torch.meshgrid(r, r, r, indexing='ij')\n"
+            "f = torch.clamp((torch.sqrt(x * x + y * y + z * z) - 0.5) / 0.1, -1, 1).contiguous()\n"
+            "vol = kf.kernel.volume(f, torch.zeros_like(f), 2.0, 0.1)\n"
+            "ik = np.linalg.inv(np.array([[400, 0, w / 2], [0, 400, h / 2], [0, 0, 1]], float)).astype(np.float32)\n"
+            "pose = np.eye(4, dtype=np.float32)\npose[2, 3] = -2\n"
+            "out = [[torch.full((h, w, 4), 7.0, device='cuda') for _ in range(2)] for _ in range(2)]\n"
+            "side, other, hit = torch.cuda.Stream(), torch.cuda.Stream(), torch.zeros(1, device='cuda')\n"
+            "def cast(maps, stream):\n"
+            "    p = [ctypes.c_void_p(m.data_ptr()) for m in maps]\n"
+            "    return kf.lib.kf_raycast(ctypes.byref(vol), kf.to_colmajor(pose), kf.to_colmajor(ik), p[0], w, h, p[1],\n"
+            "                             w, h, 0.4, 6.0, 1.99, 0.1, ctypes.c_void_p(stream), None)\n"
+            "torch.cuda.synchronize()\ng = torch.cuda.CUDAGraph()\n"
+            "with torch.cuda.graph(g, stream=side, capture_error_mode=%r):\n"
+            "    hit.add_(1)\n    assert cast(out[0], other.cuda_stream) == 0\n"
+            "g.replay()\nassert cast(out[1], 0) == 0\ntorch.cuda.synchronize()\n"
+            "assert float(hit) == 1 and all(torch.equal(a, b) for a, b in zip(*out))\n"
+            "assert float((out[0][0][..., 3] == -1).float().mean()) > 0.05\n"
+            % ([os.path.dirname(os.path.dirname(os.path.abspath(kf.__file__)))], mode))
+    r = subprocess.run([sys.executable, "-c", prog], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
