@@ -451,9 +451,9 @@ kf_status kf_session_stage_times(kf_session* s, float ms[4]);
 /* KF_DEBUG_COUNTERS makes the raycast count its work in every step (kernels built with the
  * counts; the plain kernels run otherwise): kf_session_debug_counts / kf_batch_debug_counts
  * return, for the last step, [0] rays that marched, [1] samples evaluated during large steps,
- * [2] during small steps, [3] cell skips, [4] samples the skips jumped over, [5] gradient
- * samples, [6] rays handed to the long-ray warp kernel, [7] that kernel's warp rounds.  The
- * counts cost time; results are the same. */
+ * [2] during small steps, [3] cell skips, [4] samples that skips and depth ranges jumped over,
+ * [5] gradient samples, [6] rays handed to the long-ray warp kernel, [7] that kernel's warp
+ * rounds.  The counts cost time; results are the same. */
 #define KF_DEBUG_COUNTERS 4
 #define KF_RAY_COUNTS 8
 kf_status kf_session_set_debug(kf_session* s, int flags);

@@ -39,13 +39,17 @@ namespace kf {
 
 constexpr int kMaxMarchSamples = 1 << 16;
 // loop iterations a lane marches before queueing the ray: a short budget keeps the tail of a
-// single session's frame short; steps of many sessions hand off fewer rays with a longer one
+// single session's frame short; steps of many sessions hand off fewer rays with a longer one.
+// Measured, us: a frame of a 640x480 stream in 512^3 f32 193 with a budget of 24, 189 with 40, 199 with
+// 64; 24 sessions of f16+u16 2,260 with 40, 2,243 with 64, 2,270 with 96.  The kernel's two forms go with
+// the same line: 3 blocks per SM 189 and 2,405, 4 blocks 193 and 2,246 (320x240 in 128^3 118 and 129).
 constexpr int kSerialBudgetSingle = 40;
 constexpr int kSerialBudgetMany = 64;
 constexpr int kManyRayTiles = 25000;   // more ray tiles than this in a step: kSerialBudgetMany
-// skippable super-bricks one skip may cross: 4 cuts the raycast's thread instructions by a
-// third and is 8 % faster for 32 sessions; longer runs hold a lane's warp too long (a single
-// session is 4 % slower at 8, 7 % at 16)
+// skippable super-bricks one skip may cross.  Where no depth range starts a ray, free space is crossed by
+// skips alone, and 4 cut the raycast's thread instructions by a third (32 sessions +8 %).  With the
+// ranges, us: the stream's frame 189 at 1 and 4, 192 at 8 and 16; the 24 sessions 2,249, 2,243, 2,255
+// and 2,261.
 constexpr int kRunCells = 4;
 
 bool many_ray_tiles(int ray_tiles) { return ray_tiles > kManyRayTiles; }
@@ -1051,7 +1055,7 @@ cudaError_t launch_count_tails(const EngineView& v, cudaStream_t st) {
 // long rays by whole warps.  Bound by that read (HBM) and then by the march's instructions.  One
 // thread per ray without skipping, as the reference marches, was bound by its longest rays (about
 // 2,800 samples one after another): 640 x 480 rays in 512^3 f32 took 732 us in the kernel, now
-// 180; kf_render's on a session's bounds 427 us, now about 200.
+// 168 in five (bounds 66, rays 58, long rays 31); kf_render's on a session's bounds 427 us, now 118.
 
 struct RayStage {
     float m[9];      // R K^-1 (column-major)
@@ -1232,9 +1236,13 @@ __global__ void raycast_stage_kernel(SessionDev S, RayStage rs, int w, int h) {
 
 // Bounds cost a read of the visible volume whatever the image, and the march without them costs in
 // proportion to the rays, in volumes of every size (a finer volume has more samples per ray).  Both
-// ways measured, us, image x volume, without / with bounds: 320x240 in 128^3 f32 45 / 58, in 256^3
-// 69 / 79, in 512^3 138 / 166; 640x480 in 128^3 73 / 75, in 256^3 111 / 102, in 512^3 210 / 179
-// (f16 202 / 148).  The line lies between the two images.
+// ways measured with cold caches, us, without / with bounds, in 64^3, 128^3, 256^3 and 512^3 f32:
+//   320x240   44 / 48    60 / 58    79 / 89   130 / 179
+//   400x300   44 / 48    63 / 62    81 / 91   142 / 175
+//   480x360   48 / 52    73 / 71    93 / 93   183 / 181
+//   640x480   57 / 62    99 / 87   121 / 101  245 / 181
+// (512^3 f16: 400x300 137 / 141, 480x360 180 / 146.)  The line lies between the middle two images; in
+// 64^3 it costs 4 us, in 128^3 it gives away 2.
 constexpr long long kBoundsRays = 160000;
 
 // A depth range that begins behind the camera has no bounds: the frustum's planes and the depth ranges
@@ -1245,8 +1253,9 @@ bool stage_raycast_builds_bounds(const kf_volume* vol, int w, int h, float min_d
 }
 
 // Without bounds a lane's budget is short for small images, whose few warps leave the GPU idle
-// while a lane marches (80x60 in 512^3 f32: 53 us at 24, 63 at 64), and long enough to reach most
-// surfaces for larger ones (320x240 in 512^3 f32: 203 us at 24, 138 at 64).
+// while a lane marches (512^3 f32, cold caches: 80x60 76 us at 24, 106 at 64, 160x120 90 and 111), and
+// long enough to reach most surfaces for larger ones (320x240 165 and 130, 400x300 222 and 142; in 128^3,
+// whose rays are short, 44 and 60, 52 and 63).
 static int budget_without_bounds(int w, int h) { return (long long)w * h <= 24000 ? 24 : 64; }
 
 // Every ray of a march without bounds may outlast its budget, and a ray that finds the queue full

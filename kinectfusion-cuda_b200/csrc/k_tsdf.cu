@@ -20,10 +20,10 @@
 // for one 640x480 frame into 512^3 f32 and 824 us for 24 into 512^3 f16+u16; 8^3 bricks, which fit the
 // surface best but put every access on 16 lines, 39 and 671; halves with their slices across the lanes
 // (8 lines an access, and gathers that fall on two or three image rows) 30 and 530.
-// Each 8^3 brick keeps a lower bound of its distances (an atomic minimum of every value
-// fusion stores), widened to the 2 x 2 x 2 bricks a trilinear sample can touch and to 32^3
-// super-bricks; fusion lowers the widened bounds itself whenever a brick's bound falls, so no
-// pass recomputes them.  The raycaster skips samples whose bound proves they cannot matter.
+// Each 8^3 brick keeps a lower bound of its distances (an atomic minimum: values that fusion stores
+// below one of the raycast's two thresholds lower it to one of two levels), widened to the 2 x 2 x 2
+// bricks a trilinear sample can touch and to 32^3 super-bricks; fusion lowers the widened bounds itself
+// whenever a brick's bound falls, so no pass recomputes them.  The raycaster skips samples whose bound proves they cannot matter.
 #include "kf_host.h"
 
 namespace kf {
@@ -62,8 +62,7 @@ __device__ __forceinline__ void lower_brick_bound(const FuseCtx& c, int bx, int 
 }
 
 // The approximate reciprocal.  a * rcp_approx(b) has the bits of __fdividef(a, b) for every b that is
-// not denormal (compared over 4 M pairs), without that function's scaling of denormal divisors; depths
-// above kMinDepth and sums with their reciprocals are none.
+// not denormal (compared over 4 M pairs); depths above kMinDepth and sums with their reciprocals are none.
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -591,7 +590,7 @@ cudaError_t launch_rebuild_bricks(const void* f, int fmt, int n, int* bmin, int*
 // by the queue's row updates, as a session's fusion.  One launch whose warps each tested and fused
 // 32 consecutive blocks, without the maxima, was bound by the few warps that held the frustum's
 // blocks: 808 us in the kernel at 640 x 480 into 512^3 f32, and up to 1 ms more per call in
-// cudaMalloc and cudaFree; the call now takes 83 us.
+// cudaMalloc and cudaFree; the call now takes 75 us, 41 of them kernels.
 
 // the scratch of one call, carved from one allocation
 struct StageFuseScratch {

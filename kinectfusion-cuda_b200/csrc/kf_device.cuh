@@ -94,9 +94,10 @@ struct SessionDev {
     void* tw;              // weight array (float or uint16)
     const float* xs;       // voxel-centre x (= y) coordinates, n floats
     const float* zs;       // voxel-centre z coordinates accumulated as the reference does
-    // 8^3-voxel bricks: a lower bound of the brick's distances (order-preserving int keys,
-    // kept by fusion with atomic minima) and the same widened to the 2 x 2 x 2 bricks a
-    // trilinear sample can touch, which the raycaster reads to skip samples
+    // 8^3-voxel bricks: a lower bound of the brick's distances (order-preserving int keys: exact
+    // minima after a load, lowered by fusion to one of two levels with atomic minima) and the same
+    // widened to the 2 x 2 x 2 bricks a trilinear sample can touch, which the raycaster reads to skip
+    // samples
     int* bmin;
     int* bdil;
     int* sdil;             // the same for 32^3 super-bricks (bricks [4s, 4s + 4] per axis)

@@ -106,10 +106,10 @@ constexpr int kIcpMaxPasses = 64;     // hard cap on ICP passes per frame
 
 // launch helpers (each returns the CUDA error of its launch)
 cudaError_t launch_preprocess(const EngineView& v, int grid, cudaStream_t st);
-// many: a step of more than kManyRayTiles ray tiles (serial_budget's rule)
 // The depth ranges of a step's raycast (a grid of one thread per fusion unit, or grid-stride); also
 // clears the wait record and the counters.
 cudaError_t launch_ray_range(const EngineView& v, int grid, cudaStream_t st);
+// many: a step of more than kManyRayTiles ray tiles (serial_budget's rule)
 cudaError_t launch_raycast(const EngineView& v, int grid, int fmt, cudaStream_t st, bool many);
 // debug mode: the traces of rays without a hit count the samples that depth ranges left out
 cudaError_t launch_count_tails(const EngineView& v, cudaStream_t st);
